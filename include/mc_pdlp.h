@@ -120,7 +120,8 @@ typedef struct mc_pdlp_options {
 } mc_pdlp_options;
 
 enum {
-    MC_KERNEL_PRIMAL = 0,    /* A^T y SpMV + primal prox + averages           */
+    MC_KERNEL_PRIMAL = 0,    /* A^T y SpMV + primal prox + averages; small LPs: the
+                                persistent kernel (whole restart chunks)      */
     MC_KERNEL_DUAL = 1,      /* A x-bar SpMV + dual prox + averages           */
     MC_KERNEL_DUAL_STEP = 2, /* A x-bar and A dx SpMV on step-size iterations */
     MC_KERNEL_RESIDUAL = 3,  /* KKT residual SpMVs + reductions + restart     */

@@ -62,7 +62,8 @@ struct DevState {
     int nonfinite;                  // a residual pass saw NaN/Inf
     int active_tiles[2];            // batch poll state: running column / row tiles
     int cert;                       // batch: MC_CERT_* kind when status is infeasible
-    int pad[3];
+    int fault;                      // a wait of the persistent kernel timed out
+    int pad[2];
 };
 
 // ---- cache policy helpers -------------------------------------------------

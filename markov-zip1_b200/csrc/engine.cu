@@ -6,7 +6,8 @@
 //   3. build CSR(A) from CSC(A) on the device, rows in ascending column order;
 //   4. Ruiz equilibration of both copies (ruiz_scaling.cpp:152-247);
 //   5. norms, step sizes and the starting point;
-//   6. the PDHG loop in chunks of restart_every iterations, each chunk one
+//   6. the PDHG loop in chunks of restart_every iterations: small LPs in one
+//      persistent kernel over many chunks (persist.cuh), larger ones each chunk one
 //      CUDA graph replay (2 fused SpMV kernels per iteration plus the
 //      step-size probe every 10th iteration, then the KKT residual pass and
 //      the restart logic, all on the device); the host polls one flag per

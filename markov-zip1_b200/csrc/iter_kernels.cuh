@@ -294,21 +294,22 @@ __global__ void __launch_bounds__(kBlock) k_dual_probe(Iterates<T> P) {
 }
 
 // Step-size iteration, part 2: the adaptive eta rule (pdlp.cpp:207-219).
+__device__ __forceinline__ double next_eta(double eta, double dx_norm_sq, double adx_norm_sq) {
+    if (!(dx_norm_sq > 1e-14 && adx_norm_sq > 1e-14)) return eta;
+    const double L = sqrt(adx_norm_sq / dx_norm_sq);
+    if (!(L > 1e-6)) return eta;
+    const double target = 0.95 / L;
+    if (target < eta) return maxv(0.1, maxv(target, eta * 0.8));
+    if (target > 1.05 * eta && eta < 0.99) return minv(0.99, eta * 1.05);
+    return eta;
+}
 __global__ void k_step_size(double* __restrict__ partials, int nprimal, int ndual, DevState* __restrict__ st,
                             Controls ctl) {
     __shared__ double scratch[32];
     if (st->done) return;
     const double dx_norm_sq = reduce_partials(partials + SLOT_DX * kMaxPartials, nprimal, scratch, OpSum());
     const double adx_norm_sq = reduce_partials(partials + SLOT_ADX * kMaxPartials, ndual, scratch, OpSum());
-    if (threadIdx.x == 0 && ctl.adaptive_step && dx_norm_sq > 1e-14 && adx_norm_sq > 1e-14) {
-        const double L = sqrt(adx_norm_sq / dx_norm_sq);
-        if (L > 1e-6) {
-            const double target = 0.95 / L;
-            const double eta = st->eta;
-            if (target < eta) st->eta = maxv(0.1, maxv(target, eta * 0.8));
-            else if (target > 1.05 * eta && eta < 0.99) st->eta = minv(0.99, eta * 1.05);
-        }
-    }
+    if (threadIdx.x == 0 && ctl.adaptive_step) st->eta = next_eta(st->eta, dx_norm_sq, adx_norm_sq);
 }
 
 // Step-size iteration, part 3: the dual update from the kept A x-bar.
@@ -457,28 +458,21 @@ struct TraceBuf {
     int* restarted;
 };
 
-// Restart check (pdlp.cpp:229-261): KKT scalars, termination, adaptive
-// restart, primal weight.  `span` = iterations in the chunk just finished;
-// `final_pass` = evaluate only (loop exhausted, :263-275).
-__global__ void k_finalize(double* __restrict__ partials, int nrow_parts, int ncol_parts, long long span,
-                           int final_pass, double offset, Controls ctl, TraceBuf tr,
-                           DevState* __restrict__ st) {
-    __shared__ double scratch[32];
-    if (st->done) return;
-    const double row_max = reduce_partials(partials + SLOT_ROW_MAX * kMaxPartials, nrow_parts, scratch, OpMax());
-    const double row_dobj = reduce_partials(partials + SLOT_ROW_DOBJ * kMaxPartials, nrow_parts, scratch, OpSum());
-    const double col_max = reduce_partials(partials + SLOT_COL_MAX * kMaxPartials, ncol_parts, scratch, OpMax());
-    const double col_dres = reduce_partials(partials + SLOT_COL_DRES * kMaxPartials, ncol_parts, scratch, OpSum());
-    const double col_pobj = reduce_partials(partials + SLOT_COL_POBJ * kMaxPartials, ncol_parts, scratch, OpSum());
-    const double col_dobj = reduce_partials(partials + SLOT_COL_DOBJ * kMaxPartials, ncol_parts, scratch, OpSum());
-    const double bad_rows = reduce_partials(partials + SLOT_NAN * kMaxPartials, nrow_parts, scratch, OpSum());
-    const double bad_cols = reduce_partials(partials + SLOT_NAN * kMaxPartials + kMaxPartials / 2, ncol_parts,
-                                            scratch, OpSum());
-    if (threadIdx.x != 0) return;
-    const double primal = maxv(row_max, col_max);
-    const double dual = sqrt(col_dres) / st->c_scale;
-    const double pobj = offset + col_pobj;
-    const double dobj = (offset + row_dobj) + col_dobj;
+// The sums and maxima of a residual pass over all rows and columns.
+struct CheckSums {
+    double row_max, row_dobj, bad_rows, col_max, col_dres, col_pobj, col_dobj, bad_cols;
+};
+
+// Restart check (pdlp.cpp:229-261) on the state, by one thread: KKT scalars,
+// termination, adaptive restart, primal weight.  `span` = iterations in the
+// chunk just finished; `final_pass` = evaluate only (loop exhausted,
+// :263-275).  Returns whether the solve restarts to the average.
+__device__ inline bool apply_check(DevState* st, const CheckSums& q, long long span, int final_pass, double offset,
+                                   const Controls& ctl) {
+    const double primal = maxv(q.row_max, q.col_max);
+    const double dual = sqrt(q.col_dres) / st->c_scale;
+    const double pobj = offset + q.col_pobj;
+    const double dobj = (offset + q.row_dobj) + q.col_dobj;
     const double gap = fabs(pobj - dobj) / (1.0 + fabs(pobj) + fabs(dobj));
     const double score = maxv(maxv(primal, dual), gap);
     st->primal_infeas = primal;
@@ -488,10 +482,9 @@ __global__ void k_finalize(double* __restrict__ partials, int nrow_parts, int nc
     st->dual_objective = dobj;
     st->score = score;
     st->restart_pending = 0;
-    const long long iter = st->iter + span;
     const long long isr = st->iters_since_restart + span;
-    int restarted = 0;
-    if (bad_rows + bad_cols > 0.0 || !isfinite(score)) {
+    bool restarted = false;
+    if (q.bad_rows + q.bad_cols > 0.0 || !isfinite(score)) {
         // non-finite iterates: numerical_failure (the reference would run on to
         // its iteration limit on NaNs; stopping is the engine's extension)
         st->nonfinite = 1;
@@ -515,24 +508,48 @@ __global__ void k_finalize(double* __restrict__ partials, int nrow_parts, int nc
             st->iters_since_restart = 0;
             st->last_restart_score = score;
             st->restarts += 1;
-            restarted = 1;
+            restarted = true;
         } else {
             st->avg_count += span;
             st->iters_since_restart = isr;
         }
     }
-    st->iter = iter;
-    if (tr.capacity > 0 && st->checks < tr.capacity && !final_pass) {
-        const long long q = st->checks;
-        tr.iteration[q] = iter;
-        tr.primal[q] = primal;
-        tr.dual[q] = dual;
-        tr.gap[q] = gap;
-        tr.eta[q] = st->eta;
-        tr.omega[q] = st->omega;
-        tr.restarted[q] = restarted;
-    }
+    st->iter += span;
     if (!final_pass) st->checks += 1;
+    return restarted;
+}
+
+// Entry `st->checks - 1` of the trace: the check just applied.
+__device__ inline void trace_check(const TraceBuf& tr, const DevState* st, bool restarted) {
+    const long long q = st->checks - 1;
+    if (q < 0 || q >= tr.capacity) return;
+    tr.iteration[q] = st->iter;
+    tr.primal[q] = st->primal_infeas;
+    tr.dual[q] = st->dual_infeas;
+    tr.gap[q] = st->gap;
+    tr.eta[q] = st->eta;
+    tr.omega[q] = st->omega;
+    tr.restarted[q] = restarted ? 1 : 0;
+}
+
+// The restart check of one chunk from the block partials.
+__global__ void k_finalize(double* __restrict__ partials, int nrow_parts, int ncol_parts, long long span,
+                           int final_pass, double offset, Controls ctl, TraceBuf tr,
+                           DevState* __restrict__ st) {
+    __shared__ double scratch[32];
+    if (st->done) return;
+    CheckSums q;
+    q.row_max = reduce_partials(partials + SLOT_ROW_MAX * kMaxPartials, nrow_parts, scratch, OpMax());
+    q.row_dobj = reduce_partials(partials + SLOT_ROW_DOBJ * kMaxPartials, nrow_parts, scratch, OpSum());
+    q.col_max = reduce_partials(partials + SLOT_COL_MAX * kMaxPartials, ncol_parts, scratch, OpMax());
+    q.col_dres = reduce_partials(partials + SLOT_COL_DRES * kMaxPartials, ncol_parts, scratch, OpSum());
+    q.col_pobj = reduce_partials(partials + SLOT_COL_POBJ * kMaxPartials, ncol_parts, scratch, OpSum());
+    q.col_dobj = reduce_partials(partials + SLOT_COL_DOBJ * kMaxPartials, ncol_parts, scratch, OpSum());
+    q.bad_rows = reduce_partials(partials + SLOT_NAN * kMaxPartials, nrow_parts, scratch, OpSum());
+    q.bad_cols = reduce_partials(partials + SLOT_NAN * kMaxPartials + kMaxPartials / 2, ncol_parts, scratch, OpSum());
+    if (threadIdx.x != 0) return;
+    const bool restarted = apply_check(st, q, span, final_pass, offset, ctl);
+    if (!final_pass) trace_check(tr, st, restarted);
 }
 
 // Restart to the average (pdlp.cpp:257-258): x <- x_avg, y <- y_avg.

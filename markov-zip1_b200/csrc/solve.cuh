@@ -5,11 +5,13 @@
 #include "iter_kernels.cuh"
 #include "setup_kernels.cuh"
 #include "mixed.cuh"
+#include "persist.cuh"
 
 #include <climits>
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <type_traits>
 
 namespace mc {
 
@@ -186,6 +188,164 @@ int ruiz(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const int*
     return ctx.launch_check("ruiz");
 }
 
+// ------------------------------------------------------ persistent kernel
+// The persistent form of one solve's loop (persist.cuh), when its size has one.
+struct Persist {
+    int blocks = 0;        // 0: the streaming kernels run the loop
+    bool cluster = false;  // one cluster of `blocks`, else one block per SM
+    int threads = 0;       // per block
+    int smem = 0;          // dynamic shared memory per block
+    unsigned* counter = nullptr;
+    void *tx = nullptr, *ty = nullptr;  // grid form: tagged (x-bar, dx) pairs and y
+    bool stage_y = false;  // grid form: y goes through shared memory
+    Tagged<double>*ax = nullptr, *ay = nullptr, *tp = nullptr;  // grid form: tagged averages and block partials
+};
+
+constexpr int kClusterThreads = 512, kGridThreads = 512, kGridThreadsWide = 768;
+
+template <class T>
+using PersistKernel = void (*)(Iterates<T>, MixedState, PersistArgs);
+
+inline cudaLaunchConfig_t persist_config(const Ctx& ctx, const Persist& pk, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)pk.blocks);
+    cfg.blockDim = dim3((unsigned)pk.threads);
+    cfg.dynamicSmemBytes = (size_t)pk.smem;
+    cfg.stream = ctx.stream;
+    if (pk.cluster) {
+        attr->id = cudaLaunchAttributeClusterDimension;
+        attr->val.clusterDim.x = (unsigned)pk.blocks;
+        attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    } else {
+        attr->id = cudaLaunchAttributeCooperative;
+        attr->val.cooperative = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// The form for a problem of this size.  Both forms want one line per group of
+// lanes and thread, so their reach is set by lines times lanes.  Measured on
+// B200, us per iteration (streaming kernels / cluster / grid), FP64:
+//   61 x 149, 600 entries         7.0 / 1.6 / 3.3
+//   1000 x 3000, 18k              8.5 / 4.0 / 4.0
+//   2000 x 6000, 36k              8.9 / 6.3 / 4.1     (FP32: 8.1 / 5.0 / 4.1)
+//   480 x 53k (transport), 106k  10.1 /  -  / 5.7
+//   4001 x 12k, 108k             10.0 /  -  / 5.5
+//   20k x 50k, 400k              11.9 /  -  / 7.9
+// The cluster form pays for every entry of x-bar and y that it copies to every
+// block (kClusterVector is where the grid form overtakes it); the grid form
+// pays two trips to L2 per phase and for the hottest lines of a vector that
+// everyone polls, so a short y is copied to shared memory by each block
+// (stage_y), and it is left out
+//   * for a short x-bar (rows gather few columns: 30000 x 3000 took 12 us
+//     against 10.6), and
+//   * for rows of so few entries that one lane takes a row: its trips to L2
+//     then follow one another (60000 x 50000, 5 per row: 18 us against 11).
+constexpr int kClusterVector64 = 4096, kClusterVector32 = 6400;  // n + m
+template <class T>
+int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned* counter, void* tagged, Persist* out) {
+    *out = Persist{};
+    int dev_smem = 0;
+    CU(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
+    const int top = dev_smem - 4096;  // less the kernel's static arrays
+    // a block holds at most one line per group of lanes
+    auto lanes_of = [&](long long blocks) {
+        return std::max((n + blocks - 1) / blocks * pl.g_col, (m + blocks - 1) / blocks * pl.g_row);
+    };
+    auto whole_warps = [&](long long blocks) { return (int)std::max<long long>(64, (lanes_of(blocks) + 31) / 32 * 32); };
+    // shared memory of a block: the matrix slices, with a margin for uneven
+    // shares (a slice that does not fit stays in global memory), and `vectors`
+    auto need = [&](int blocks, double vectors) {
+        return std::min<double>(top, vectors + 1.5 * 2.0 * (4 + sizeof(T)) * (double)nnz / blocks + 1024.0);
+    };
+    if ((long long)n + m <= (sizeof(T) == 8 ? kClusterVector64 : kClusterVector32)) {
+        PersistKernel<T> ck = k_persist<T, true, kClusterThreads>;
+        int c = 1;
+        while (c < 16 && lanes_of(c) > kClusterThreads) c *= 2;
+        if (lanes_of(c) <= kClusterThreads) {
+            CU(cudaFuncSetAttribute(ck, cudaFuncAttributeMaxDynamicSharedMemorySize, top));
+            CU(cudaFuncSetAttribute(ck, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            Persist pk;
+            pk.cluster = true;
+            pk.counter = counter;
+            pk.blocks = c;
+            pk.threads = whole_warps(c);
+            pk.smem = (int)need(c, sizeof(T) * (2.0 * n + m));
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = persist_config(ctx, pk, &attr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, ck, &cfg) == cudaSuccess && clusters > 0) {
+                *out = pk;
+                return MC_OK;
+            }
+            cudaGetLastError();  // no room for this cluster: the grid form, or the streaming kernels
+        }
+    }
+    const int nb = ctx.sm_count;
+    if (tagged && nb <= kPersistMaxBlocks && lanes_of(nb) <= kGridThreadsWide && pl.g_row >= 2 &&
+        (double)n * nb > 2.0 * (double)nnz) {
+        Persist pk;
+        pk.blocks = nb;
+        pk.threads = whole_warps(nb);
+        pk.counter = counter;
+        pk.ax = static_cast<Tagged<double>*>(tagged);
+        pk.ay = pk.ax + n;
+        pk.tp = pk.ay + m;
+        pk.tx = pk.tp + kPersistPartials;
+        pk.ty = static_cast<Tagged<T>*>(pk.tx) + 2LL * n;
+        PersistKernel<T> gk = pk.threads <= kGridThreads ? k_persist<T, false, kGridThreads>
+                                                         : k_persist<T, false, kGridThreadsWide>;
+        CU(cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, top));
+        pk.stage_y = m * (double)nb <= 2.0 * (double)nnz && 2.0 * m * sizeof(T) <= 65536.0;
+        pk.smem = (int)need(nb, pk.stage_y ? 2.0 * m * sizeof(T) : 0.0);
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gk, pk.threads, (size_t)pk.smem) == cudaSuccess &&
+            per_sm > 0)
+            *out = pk;
+        else cudaGetLastError();
+    }
+    return MC_OK;
+}
+
+// One launch: `chunks` whole chunks, then (with final_pass) `rem` iterations
+// and the final evaluation.
+template <class E>
+int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int rem, int final_pass, const Controls& ctl,
+                   const TraceBuf& tr) {
+    using T = std::remove_pointer_t<decltype(eng.P.x)>;
+    const Persist& pk = eng.pk;
+    PersistArgs A{};
+    A.O = eng.O;
+    A.ctl = ctl;
+    A.tr = tr;
+    A.chunks = chunks;
+    A.R = (int)R;
+    A.rem = rem;
+    A.final_pass = final_pass;
+    A.g_col = eng.pl.g_col;
+    A.g_row = eng.pl.g_row;
+    A.g_probe = eng.pl.g_probe;
+    A.smem_bytes = pk.smem;
+    A.counter = pk.counter;
+    A.tx = pk.tx;
+    A.ty = pk.ty;
+    A.stage_y = pk.stage_y;
+    A.ax = pk.ax;
+    A.ay = pk.ay;
+    A.tp = pk.tp;
+    if (!pk.cluster) CU(cudaMemsetAsync(pk.counter, 0, sizeof(unsigned), ctx.stream));
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = persist_config(ctx, pk, &attr);
+    ctx.begin_launch(MC_KERNEL_PRIMAL);
+    if (pk.cluster) CU(cudaLaunchKernelEx(&cfg, k_persist<T, true, kClusterThreads>, eng.P, eng.M, A));
+    else if (pk.threads <= kGridThreads) CU(cudaLaunchKernelEx(&cfg, k_persist<T, false, kGridThreads>, eng.P, eng.M, A));
+    else CU(cudaLaunchKernelEx(&cfg, k_persist<T, false, kGridThreadsWide>, eng.P, eng.M, A));
+    ctx.end_launch();
+    return ctx.launch_check("persistent kernel");
+}
+
 // ------------------------------------------------------- iteration chunks
 // One precision's way of enqueuing iterations and restart checks.  FP64 runs
 // the fused kernels on the iterate itself; the mixed form runs the FP32
@@ -196,8 +356,10 @@ struct Engine64 {
     void use_class(int) const {}
 
     Iterates<double> P;
+    MixedState M{};  // unused: the persistent kernel takes one for both forms
     Original O;
     Plan pl;
+    Persist pk;
 
     int iteration(Ctx& ctx, int k, bool step, const Controls& ctl) const {
         cudaStream_t s = ctx.stream;
@@ -256,6 +418,7 @@ struct EngineMixed {
     MixedState M;
     Original O;
     Plan pl;
+    Persist pk;
     int nb_res_row = 1, nb_res_col = 1, nb_recenter = 1, nb_apply = 1;
 
     int iteration(Ctx& ctx, int k, bool step, const Controls& ctl) const {
@@ -369,6 +532,44 @@ struct ChunkLoop {
     long long recipe[40][MC_KERNEL_KINDS] = {};
 };
 
+template <class E, class = void>
+struct has_persist : std::false_type {};
+template <class E>
+struct has_persist<E, std::void_t<decltype(std::declval<E&>().pk)>> : std::true_type {};
+
+// loop_chunks on the persistent kernel: kPersistChunks chunks per launch
+// (a few milliseconds, so that a long solve is polled and never holds the
+// device in one launch), the host polling one launch behind.
+constexpr int kPersistChunks = 32;
+template <class E>
+int loop_persist(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long stop, long long R,
+                 const Controls& ctl, const TraceBuf& tr) {
+    cudaStream_t s = ctx.stream;
+    while (L.chunk < stop && !L.done) {
+        const int chunks = (int)std::min<long long>(stop - L.chunk, std::max<long long>(1, kPersistChunks * 40 / R));
+        TRY(launch_persist(ctx, eng, chunks, R, 0, 0, ctl, tr));
+        TRY(ctx.drain_profile());
+        L.chunk += chunks;
+        L.base += chunks * R;
+        if (L.have_prev) {
+            CU(cudaEventSynchronize(ctx.ev_poll[L.ev_idx ^ 1]));
+            if (ctx.h_state[L.ev_idx ^ 1].done || ctx.h_state[L.ev_idx ^ 1].fault) L.done = true;
+        }
+        if (L.chunk < stop && !L.done) {
+            CU(cudaMemcpyAsync(&ctx.h_state[L.ev_idx], st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+            CU(cudaEventRecord(ctx.ev_poll[L.ev_idx], s));
+            L.have_prev = true;
+            L.ev_idx ^= 1;
+        }
+    }
+    CU(cudaMemcpyAsync(&ctx.h_state[2], st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
+    L.have_prev = false;
+    if (ctx.h_state[2].fault) return set_error(MC_ERR_CUDA, "a wait of the persistent kernel timed out");
+    if (ctx.h_state[2].done) L.done = true;
+    return MC_OK;
+}
+
 // Enqueue up to `max_chunks` further chunks (each a CUDA graph replay), the
 // host polling the device state one chunk group behind, so that the GPU never
 // idles between chunks.  Returns with the stream synchronised and the state
@@ -378,6 +579,9 @@ int loop_chunks(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long ma
                 int poll_every, const Controls& ctl, const TraceBuf& tr) {
     cudaStream_t s = ctx.stream;
     const long long stop = L.chunk + std::min(max_chunks, L.full_chunks - L.chunk);
+    if constexpr (has_persist<E>::value) {
+        if (eng.pk.blocks > 0) return loop_persist(ctx, eng, st, L, stop, R, ctl, tr);
+    }
     for (; L.chunk < stop && !L.done; ++L.chunk) {
         eng.use_class(L.cls);
         if (ctx.profiling) {
@@ -429,6 +633,14 @@ int finish_chunks(Ctx& ctx, const E& eng, const ChunkLoop& L, long long maxit, l
     if (!L.done && L.chunk == L.full_chunks) {
         const long long rem = maxit - L.full_chunks * R;
         if (rem > 0 || L.full_chunks == 0) {
+            if constexpr (has_persist<E>::value) {
+                if (eng.pk.blocks > 0) {
+                    TRY(launch_persist(ctx, eng, 0, R, (int)rem, 1, ctl, tr));
+                    TRY(ctx.drain_profile());
+                    CU(cudaStreamSynchronize(ctx.stream));
+                    return MC_OK;
+                }
+            }
             TRY(enqueue_span(ctx, eng, L.base, 0, (int)rem, ctl));
             TRY(eng.check(ctx, rem, 1, ctl, tr));
             TRY(ctx.drain_profile());
@@ -624,6 +836,10 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
     for (auto& v : o_m) v = L.add<double>(m);
     const size_t o_partials = L.add<double>((long long)NUM_SLOTS * kMaxPartials);
     const size_t o_state = L.add<DevState>(1);
+    const size_t o_counter = L.add<unsigned>(1);
+    // the persistent kernel's grid form: tagged averages, block partials, x-bar, dx and y
+    const bool small = std::max(n, m) <= kPersistMaxBlocks * kGridThreadsWide;
+    const size_t o_tagged = small ? L.add<Tagged<double>>(3LL * n + 3LL * m + kPersistPartials) : 0;
     // (x-bar, dx) pairs of the step-size iterations, in the iterate type
     const size_t o_xdx = mixed ? L.add<float>(2LL * n) : L.add<double>(2LL * n);
     const size_t o_tr_it = L.add<long long>(trace_cap);
@@ -794,6 +1010,8 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         P.st = st;
         eng.O = O;
         eng.pl = make_plan<double>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
+        TRY(plan_persist<double>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
+                            o_tagged ? at(o_tagged) : nullptr, &eng.pk));
         TRY(choose_start(ctx, eng, st, ctl, have_warm, o->warm_start_guard != 0, start, [] { return MC_OK; }, res));
     } else {
         EngineMixed& eng = SS.emx;
@@ -876,6 +1094,8 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         M.yb = f_yb;
         eng.O = O;
         eng.pl = make_plan<float>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
+        TRY(plan_persist<float>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
+                            o_tagged ? at(o_tagged) : nullptr, &eng.pk));
         // the FP32 dual kernel has no block partials: one block per kBlock/G rows
         // (about 40 waves) lets the block scheduler even out the last wave,
         // 13% faster on B200 than one resident wave; the FP64 and primal
