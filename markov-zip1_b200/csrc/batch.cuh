@@ -556,37 +556,14 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     // ---- setup: transpose, Ruiz per LP, data per LP
     TRY(build_csr(ctx, (int)m, (int)n, nnz, cs, ri, cv, rs, ci, rv, static_cast<int*>(at(o_cursor)),
                   static_cast<int*>(at(o_long)), counters, static_cast<int*>(at(o_scan))));
-    ctx.begin_launch(MC_KERNEL_SETUP);
-    k_fill<double><<<blocks_for(ctx, m, kBlock), kBlock, 0, s>>>(row_scale, m, 1.0);
-    ctx.end_launch();
-    ctx.begin_launch(MC_KERNEL_SETUP);
-    k_fill<double><<<blocks_for(ctx, n, kBlock), kBlock, 0, s>>>(col_scale, n, 1.0);
-    ctx.end_launch();
-    double* r_tmp = y_work[2];
-    double* c_tmp = x_work[3];
-    const long long passes = o->ruiz_scaling ? o->ruiz_iterations : 0;
-    for (long long pass = 0; pass < passes && nnz > 0; ++pass) {
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_line_max<<<nct, kBlock, 0, s>>>(cs, cv, c_tmp, partials, SLOT_A, B.cols, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_line_max<<<nrt, kBlock, 0, s>>>(rs, rv, r_tmp, partials, SLOT_B, B.rows, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_check<<<count, 256, 0, s>>>(partials, B, 1e-3);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_deltas<<<nrt, kBlock, 0, s>>>(r_tmp, row_scale, B.rows, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_deltas<<<nct, kBlock, 0, s>>>(c_tmp, col_scale, B.cols, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_rescale<<<nct, kBlock, 0, s>>>(cs, ri, cv, c_tmp, r_tmp, B.cols, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        kb_ruiz_rescale<<<nrt, kBlock, 0, s>>>(rs, ci, rv, r_tmp, c_tmp, B.rows, st);
-        ctx.end_launch();
+    {
+        RuizSide C = ruiz_side_of((int)n, nnz, cs, ri, cv, col_scale, x_work[3], col_norm);
+        RuizSide R = ruiz_side_of((int)m, nnz, rs, ci, rv, row_scale, y_work[2], row_norm);
+        C.lanes = gc;  // the tiles' lanes
+        R.lanes = gr;
+        C.lp = B.cols.lp, C.l0 = B.cols.l0, C.l1 = B.cols.l1, C.ntiles = nct;
+        R.lp = B.rows.lp, R.l0 = B.rows.l0, R.l1 = B.rows.l1, R.ntiles = nrt;
+        TRY(launch_ruiz(ctx, C, R, nnz > 0 && o->ruiz_scaling ? o->ruiz_iterations : 0, 1e-3, count, partials, st));
     }
     Iterates<double> P;
     P.m = (int)m;
@@ -777,6 +754,7 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     long long total = 0;
     for (int q = 0; q < MC_KERNEL_KINDS; ++q) total += ctx.launches[q];
     const double total_ms = now_ms() - t_begin;
+    if (hs[0].fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     for (int b = 0; b < count; ++b) {
         mc_pdlp_result& r = results[b];
         std::snprintf(r.backend_actually_used, sizeof r.backend_actually_used, "cuda");

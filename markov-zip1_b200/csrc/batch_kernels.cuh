@@ -434,63 +434,6 @@ __global__ void __launch_bounds__(kBlock) kb_restart_copy(Iterates<double> P, Ba
 }
 
 // ------------------------------------------------------------------ setup
-// Ruiz per LP: line maxima of a tile, per-LP check, deltas and rescale skip
-// LPs whose Ruiz has converged (ruiz_scaling.cpp:167-218 per LP).
-__global__ void kb_ruiz_line_max(const int* __restrict__ start, const double* __restrict__ value,
-                                 double* __restrict__ norm, double* __restrict__ partials, int slot,
-                                 TileTable T, const DevState* __restrict__ st) {
-    __shared__ double scratch[32];
-    double err = 0.0;
-    if (!st[T.lp[blockIdx.x]].ruiz_done) {
-        for (int j = T.l0[blockIdx.x] + threadIdx.x; j < T.l1[blockIdx.x]; j += blockDim.x) {
-            double mx = 0.0;
-            for (int p = start[j]; p < start[j + 1]; ++p) mx = maxv(mx, fabs(value[p]));
-            if (mx == 0.0) mx = 1.0;
-            norm[j] = mx;
-            err = maxv(err, fabs(1.0 - mx));
-        }
-    }
-    err = block_reduce(err, scratch, OpMax());
-    if (threadIdx.x == 0) partials[slot * kMaxTiles + blockIdx.x] = err;
-}
-
-__global__ void kb_ruiz_check(const double* __restrict__ partials, BatchRefs B, double tolerance) {
-    __shared__ double scratch[32];
-    const int lp = blockIdx.x;
-    DevState* st = B.st + lp;
-    if (st->ruiz_done) return;
-    const int c0 = B.cols.first[lp], nc = B.cols.first[lp + 1] - c0;
-    const int r0 = B.rows.first[lp], nr = B.rows.first[lp + 1] - r0;
-    const double c = reduce_partials(partials + SLOT_A * kMaxTiles + c0, nc, scratch, OpMax());
-    const double r = reduce_partials(partials + SLOT_B * kMaxTiles + r0, nr, scratch, OpMax());
-    if (threadIdx.x == 0) {
-        if (r < tolerance && c < tolerance) st->ruiz_done = 1;
-        else st->ruiz_passes += 1;
-    }
-}
-
-__global__ void kb_ruiz_deltas(double* __restrict__ norm, double* __restrict__ scale, TileTable T,
-                               const DevState* __restrict__ st) {
-    if (st[T.lp[blockIdx.x]].ruiz_done) return;
-    for (int j = T.l0[blockIdx.x] + threadIdx.x; j < T.l1[blockIdx.x]; j += blockDim.x) {
-        const double d = 1.0 / sqrt(norm[j]);
-        norm[j] = d;
-        scale[j] *= d;
-    }
-}
-
-__global__ void kb_ruiz_rescale(const int* __restrict__ start, const int* __restrict__ inner,
-                                double* __restrict__ value, const double* __restrict__ delta_outer,
-                                const double* __restrict__ delta_inner, TileTable T,
-                                const DevState* __restrict__ st) {
-    if (st[T.lp[blockIdx.x]].ruiz_done) return;
-    for (int j = T.l0[blockIdx.x] + threadIdx.x; j < T.l1[blockIdx.x]; j += blockDim.x) {
-        const double dout = delta_outer[j];
-        for (int p = start[j]; p < start[j + 1]; ++p)
-            value[p] = __dmul_rn(value[p], __dmul_rn(delta_inner[inner[p]], dout));
-    }
-}
-
 // Column setup of a tile (k_setup_cols per LP) plus the crossed-bound
 // certificate: a column with lower > upper makes its LP infeasible.
 __global__ void kb_setup_cols(const int* __restrict__ col_start, const double* __restrict__ value,

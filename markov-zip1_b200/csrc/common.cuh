@@ -62,7 +62,7 @@ struct DevState {
     int nonfinite;                  // a residual pass saw NaN/Inf
     int active_tiles[2];            // batch poll state: running column / row tiles
     int cert;                       // batch: MC_CERT_* kind when status is infeasible
-    int fault;                      // a wait of the persistent kernel timed out
+    int fault;                      // a wait of a cooperative kernel timed out
     int pad[2];
 };
 
@@ -137,6 +137,13 @@ __device__ __forceinline__ T group_sum(T v) {
     return v;
 }
 
+// sum over aligned groups of G lanes (the order of group_sum<G>)
+template <class T>
+__device__ __forceinline__ T group_sum_n(T v, int G) {
+    for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
 struct OpSum {
     __device__ __forceinline__ double operator()(double a, double b) const { return a + b; }
     static constexpr double identity = 0.0;
@@ -173,5 +180,49 @@ __device__ __forceinline__ double reduce_partials(const double* p, int count, do
     for (int i = threadIdx.x; i < count; i += blockDim.x) v = op(v, p[i]);
     return block_reduce(v, scratch, op);
 }
+
+constexpr unsigned kSpinLimit = 1u << 23;  // polls of one wait (seconds) before a thread gives up
+
+// Barrier across the blocks of a launch, in two halves: the hardware barrier of
+// a cluster (CL), or for a cooperative launch a counter, zeroed before it, that
+// every block adds to and one thread per block polls (2 us at 148 blocks).
+template <bool CL>
+struct BlockBarrier {
+    unsigned* counter;
+    unsigned target;
+    bool alone;  // a cluster of one block
+    __device__ __forceinline__ void arrive() {
+        if (CL) {
+            if (!alone) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            return;
+        }
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    }
+    // false once the limit is reached: the block leaves the kernel
+    __device__ __forceinline__ bool wait() {
+        if (CL) {
+            if (alone) __syncthreads();
+            else asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            return true;
+        }
+        int ok = 1;
+        if (threadIdx.x == 0) {
+            unsigned v, spins = 0;
+            do {
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+                if (v - target < (1u << 30)) break;
+                ok = ++spins < kSpinLimit;
+            } while (ok);
+            __threadfence();
+        }
+        return __syncthreads_and(ok) != 0;
+    }
+    __device__ __forceinline__ bool sync() {
+        arrive();
+        return wait();
+    }
+};
 
 }  // namespace mc

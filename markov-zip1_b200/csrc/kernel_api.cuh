@@ -136,15 +136,15 @@ int mc_ruiz_equilibrate(mc_pdlp_ctx* c, int32_t m, int32_t n, int64_t nnz, const
     cudaStream_t s = ctx->stream;
     double *r_tmp = nullptr, *c_tmp = nullptr, *partials = nullptr;
     DevState* st = nullptr;
-    CU(cudaMallocAsync(reinterpret_cast<void**>(&r_tmp), sizeof(double) * (size_t)(m + 1), s));
-    CU(cudaMallocAsync(reinterpret_cast<void**>(&c_tmp), sizeof(double) * (size_t)(n + 1), s));
+    CU(cudaMallocAsync(reinterpret_cast<void**>(&r_tmp), sizeof(double) * 2 * (size_t)(m + 1), s));
+    CU(cudaMallocAsync(reinterpret_cast<void**>(&c_tmp), sizeof(double) * 2 * (size_t)(n + 1), s));
     CU(cudaMallocAsync(reinterpret_cast<void**>(&partials), sizeof(double) * NUM_SLOTS * kMaxPartials, s));
     CU(cudaMallocAsync(reinterpret_cast<void**>(&st), sizeof(DevState), s));
     CU(cudaMemsetAsync(st, 0, sizeof(DevState), s));
     int rc = MC_OK;
     if (m > 0 && n > 0) {
         rc = ruiz(*ctx, m, n, nnz, col_start, row_index, csc_value, row_start, col_index, csr_value, row_scale,
-                  col_scale, r_tmp, c_tmp, partials, st, max_iterations);
+                  col_scale, r_tmp, r_tmp + m + 1, c_tmp, c_tmp + n + 1, partials, st, max_iterations);
         if (rc == MC_OK && objective && var_lower && var_upper && row_lower && row_upper) {
             k_ruiz_apply<<<blocks_for(*ctx, (long long)n + m, kBlock), kBlock, 0, s>>>(
                 m, n, row_scale, col_scale, objective, var_lower, var_upper, row_lower, row_upper);
@@ -161,6 +161,7 @@ int mc_ruiz_equilibrate(mc_pdlp_ctx* c, int32_t m, int32_t n, int64_t nnz, const
     TRY(rc);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(state)", __LINE__);
     CU(cudaStreamSynchronize(s));
+    if (h.fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     if (iterations_executed) *iterations_executed = h.ruiz_passes;
     return MC_OK;
 }
@@ -212,8 +213,8 @@ int mc_ruiz_equilibrate_canonical(mc_pdlp_ctx* c, int32_t m, int32_t n, int64_t 
     alloc(reinterpret_cast<void**>(&long_rows), sizeof(int) * (size_t)(m + 1));
     alloc(reinterpret_cast<void**>(&counters), sizeof(int) * 4);
     alloc(reinterpret_cast<void**>(&scan), sizeof(int) * scan_ints);
-    alloc(reinterpret_cast<void**>(&r_tmp), sizeof(double) * (size_t)(m + 1));
-    alloc(reinterpret_cast<void**>(&c_tmp), sizeof(double) * (size_t)(n + 1));
+    alloc(reinterpret_cast<void**>(&r_tmp), sizeof(double) * 2 * (size_t)(m + 1));
+    alloc(reinterpret_cast<void**>(&c_tmp), sizeof(double) * 2 * (size_t)(n + 1));
     alloc(reinterpret_cast<void**>(&partials), sizeof(double) * NUM_SLOTS * kMaxPartials);
     alloc(reinterpret_cast<void**>(&st), sizeof(DevState));
     DevState h;
@@ -235,7 +236,7 @@ int mc_ruiz_equilibrate_canonical(mc_pdlp_ctx* c, int32_t m, int32_t n, int64_t 
     if (rc == MC_OK) rc = build_csr(*ctx, m, n, nnz, col_start, row_index, value, rs, ci, rv, cursor, long_rows,
                                     counters, scan);
     if (rc == MC_OK) rc = ruiz(*ctx, m, n, nnz, col_start, row_index, value, rs, ci, rv, row_scale, col_scale, r_tmp,
-                              c_tmp, partials, st, max_iterations, tolerance);
+                              r_tmp + m + 1, c_tmp, c_tmp + n + 1, partials, st, max_iterations, tolerance);
     if (rc == MC_OK) {
         cudaMemsetAsync(counters, 0, sizeof(int) * 4, s);
         k_ruiz_canonical_finish<<<blocks_for(*ctx, (long long)m + n, kBlock), kBlock, 0, s>>>(
@@ -251,6 +252,7 @@ int mc_ruiz_equilibrate_canonical(mc_pdlp_ctx* c, int32_t m, int32_t n, int64_t 
         if (p) cudaFreeAsync(p, s);
     TRY(rc);
     CU(cudaStreamSynchronize(s));
+    if (h.fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     // the reference throws overflow_error here (ruiz_scaling.cpp:112-121)
     if (hbad & 1) return set_error(MC_ERR_INVALID_ARGUMENT, "non-finite scaled RHS");
     if (hbad & 2) return set_error(MC_ERR_INVALID_ARGUMENT, "non-finite scaled objective");

@@ -45,55 +45,6 @@ namespace mc {
 
 constexpr int kPersistMaxBlocks = 160;
 constexpr int kPersistPartials = 2 * 2 * 8 * kPersistMaxBlocks;  // tagged partials and sums of the reductions
-constexpr unsigned kSpinLimit = 1u << 23;  // polls of one wait (seconds) before a thread gives up
-
-// Barrier across the blocks of the launch, in two halves.  Grid form (once per
-// launch): a counter that every block adds to and one thread per block polls.
-template <bool CL>
-struct BlockBarrier {
-    unsigned* counter;
-    unsigned target;
-    bool alone;  // a cluster of one block
-    __device__ __forceinline__ void arrive() {
-        if (CL) {
-            if (!alone) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-            return;
-        }
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-    }
-    // false once the limit is reached: the block leaves the kernel
-    __device__ __forceinline__ bool wait() {
-        if (CL) {
-            if (alone) __syncthreads();
-            else asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-            return true;
-        }
-        int ok = 1;
-        if (threadIdx.x == 0) {
-            unsigned v, spins = 0;
-            do {
-                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-                if (v - target < (1u << 30)) break;
-                ok = ++spins < kSpinLimit;
-            } while (ok);
-            __threadfence();
-        }
-        return __syncthreads_and(ok) != 0;
-    }
-    __device__ __forceinline__ bool sync() {
-        arrive();
-        return wait();
-    }
-};
-
-// sum over aligned groups of G lanes (the order of group_sum<G>)
-template <class T>
-__device__ __forceinline__ T group_sum_n(T v, int G) {
-    for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
 
 // ---- gathered vectors
 // Grid form: an entry and the number of the iteration that wrote it, in one

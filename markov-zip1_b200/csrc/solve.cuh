@@ -148,44 +148,53 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
 }
 
 // ------------------------------------------------------------------ Ruiz
+// One cooperative launch (k_ruiz).  C, R: both copies, their tiles and the
+// scratch of their deltas; work: at least 6 nlp + 2 words of device memory.
+int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long passes, double tolerance, int nlp,
+                double* work, DevState* st) {
+    cudaStream_t s = ctx.stream;
+    unsigned long long* errs = reinterpret_cast<unsigned long long*>(work);
+    unsigned* counter = reinterpret_cast<unsigned*>(errs + 6 * (size_t)nlp);
+    CU(cudaMemsetAsync(work, 0, sizeof(double) * (6 * (size_t)nlp + 2), s));
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid_for(ctx, k_ruiz, std::max(C.ntiles, R.ntiles), 1));
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    ctx.begin_launch(MC_KERNEL_SETUP);
+    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, st));
+    ctx.end_launch();
+    return ctx.launch_check("ruiz");
+}
+
+inline RuizSide ruiz_side_of(int lines, long long nnz, const int* start, const int* inner, double* value, double* scale,
+                             double* d0, double* d1) {
+    RuizSide S{};
+    S.start = start;
+    S.inner = inner;
+    S.value = value;
+    S.scale = scale;
+    S.delta[0] = d0;
+    S.delta[1] = d1;
+    S.lanes = pick_lanes(lines > 0 ? (double)nnz / lines : 1.0);
+    S.lines = lines;
+    S.per = kBlock / S.lanes;
+    S.ntiles = (lines + S.per - 1) / S.per;
+    return S;
+}
+
+// r_d0, r_d1 [m] and c_d0, c_d1 [n]: scratch
 int ruiz(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const int* csc_row, double* csc_val,
          const int* csr_start, const int* csr_col, double* csr_val, double* row_scale, double* col_scale,
-         double* r_tmp, double* c_tmp, double* partials, DevState* st, long long passes,
+         double* r_d0, double* r_d1, double* c_d0, double* c_d1, double* partials, DevState* st, long long passes,
          double tolerance = 1e-3) {
-    cudaStream_t s = ctx.stream;
-    ctx.begin_launch(MC_KERNEL_SETUP);
-    k_fill<double><<<blocks_for(ctx, m, kBlock), kBlock, 0, s>>>(row_scale, m, 1.0);
-    ctx.end_launch();
-    ctx.begin_launch(MC_KERNEL_SETUP);
-    k_fill<double><<<blocks_for(ctx, n, kBlock), kBlock, 0, s>>>(col_scale, n, 1.0);
-    ctx.end_launch();
-    if (nnz == 0) return ctx.launch_check("ruiz");
-    const int nbc = blocks_for(ctx, n, kBlock), nbr = blocks_for(ctx, m, kBlock);
-    for (long long pass = 0; pass < passes; ++pass) {
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_line_max<<<nbc, kBlock, 0, s>>>(n, csc_start, csc_val, c_tmp, partials + SLOT_A * kMaxPartials, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_line_max<<<nbr, kBlock, 0, s>>>(m, csr_start, csr_val, r_tmp, partials + SLOT_B * kMaxPartials, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_check<<<1, 1024, 0, s>>>(partials + SLOT_B * kMaxPartials, nbr, partials + SLOT_A * kMaxPartials,
-                                        nbc, tolerance, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_deltas<<<nbr, kBlock, 0, s>>>(m, r_tmp, row_scale, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_deltas<<<nbc, kBlock, 0, s>>>(n, c_tmp, col_scale, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_rescale<<<nbc, kBlock, 0, s>>>(n, csc_start, csc_row, csc_val, c_tmp, r_tmp, 0, st);
-        ctx.end_launch();
-        ctx.begin_launch(MC_KERNEL_SETUP);
-        k_ruiz_rescale<<<nbr, kBlock, 0, s>>>(m, csr_start, csr_col, csr_val, r_tmp, c_tmp, 1, st);
-        ctx.end_launch();
-    }
-    return ctx.launch_check("ruiz");
+    return launch_ruiz(ctx, ruiz_side_of(n, nnz, csc_start, csc_row, csc_val, col_scale, c_d0, c_d1),
+                       ruiz_side_of(m, nnz, csr_start, csr_col, csr_val, row_scale, r_d0, r_d1),
+                       nnz > 0 ? passes : 0, tolerance, 1, partials, st);
 }
 
 // ------------------------------------------------------ persistent kernel
@@ -565,7 +574,7 @@ int loop_persist(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long s
     CU(cudaMemcpyAsync(&ctx.h_state[2], st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     L.have_prev = false;
-    if (ctx.h_state[2].fault) return set_error(MC_ERR_CUDA, "a wait of the persistent kernel timed out");
+    if (ctx.h_state[2].fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     if (ctx.h_state[2].done) L.done = true;
     return MC_OK;
 }
@@ -620,6 +629,7 @@ int loop_chunks(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long ma
     CU(cudaMemcpy(&ctx.h_state[2], st, sizeof(DevState), cudaMemcpyDeviceToHost));
     L.have_prev = false;  // everything enqueued has completed
     L.inflight = 0;
+    if (ctx.h_state[2].fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     if (ctx.h_state[2].done) L.done = true;
     return MC_OK;
 }
@@ -941,7 +951,7 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
                   static_cast<int*>(at(o_cursor)), static_cast<int*>(at(o_long)), counters,
                   static_cast<int*>(at(o_scan))));
     TRY(ruiz(ctx, m, n, nnz, csc_start, csc_row, csc_val, csr_start, csr_col, csr_val, row_scale, col_scale,
-             ax_bar, dx, partials, st, o->ruiz_scaling ? o->ruiz_iterations : 0));
+             ax_bar, row_norm, dx, col_norm, partials, st, o->ruiz_scaling ? o->ruiz_iterations : 0));
     const double obj_sign = (lp->objective_sense == MC_MAXIMIZE) ? -1.0 : 1.0;
     const int nbc = blocks_for(ctx, n, kBlock), nbr = blocks_for(ctx, m, kBlock);
     // starting point (pdlp.cpp:153-191): warm = the caller's warm start and

@@ -1203,7 +1203,8 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     CU(cudaMemsetAsync(st, 0, sizeof(DevState) * (count + 2), s));
     TRY(build_csr(ctx, m, n, nnz, cs, ri, cv, rs, ci, rv, static_cast<int*>(at(o_cursor)),
                   static_cast<int*>(at(o_long)), counters, static_cast<int*>(at(o_scan))));
-    TRY(ruiz(ctx, m, n, nnz, cs, ri, cv, rs, ci, rv, row_scale, col_scale, y_scratch, x_scratch, part1, st,
+    TRY(ruiz(ctx, m, n, nnz, cs, ri, cv, rs, ci, rv, row_scale, col_scale, y_scratch, row_norm, x_scratch,
+             col_norm, part1, st,
              o->ruiz_scaling ? o->ruiz_iterations : 0));
     const double obj_sign = (base->objective_sense == MC_MAXIMIZE) ? -1.0 : 1.0;
     const int nbc = blocks_for(ctx, n, kBlock), nbr = blocks_for(ctx, m, kBlock);
@@ -1393,6 +1394,7 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     CU(cudaMemcpyAsync(hcert.data(), V.cert_idx, sizeof(int) * hcert.size(), cudaMemcpyDeviceToHost, s));
     CU(cudaEventRecord(ctx.ev_d, s));
     CU(cudaStreamSynchronize(s));
+    if (hs[0].fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     TRY(ctx.drain_profile());
     float h2d = 0.f, kern = 0.f, d2h = 0.f;
     CU(cudaEventElapsedTime(&h2d, ctx.ev_a, ctx.ev_b));
