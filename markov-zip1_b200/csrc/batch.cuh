@@ -360,6 +360,7 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     const size_t o_part = L.add<double>((long long)NUM_SLOTS * kMaxTiles);
     const size_t o_st = L.add<DevState>(count + 1);
     const size_t o_off = L.add<double>(2LL * count);
+    const size_t o_offs = L.add<int>(3LL * (count + 1)), o_ends = L.add<int>(count);
     const size_t o_flags = L.add<int>(count);
     const size_t o_cert = L.add<int>(2LL * count);
     const size_t o_yprev = L.add<double>(m), o_dray = L.add<double>(m);
@@ -436,39 +437,44 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     CU(cudaEventRecord(ctx.ev_a, s));
     int* counters = static_cast<int*>(at(o_counters));
     CU(cudaMemsetAsync(counters, 0, sizeof(int) * 4, s));
+    // one kind of array after the other, so that the LPs' pieces follow one another
+    Staging& up = ctx.staging;
+    int* ends = static_cast<int*>(at(o_ends));
     for (int b = 0; b < count; ++b) {
-        const mc_lp& lp = lps[b];
-        const long long nb = lp.num_cols, mb = lp.num_rows, zb = lp.nnz;
-        CU(cudaMemcpyAsync(cs + col_off[b], lp.col_start, sizeof(int) * (size_t)(nb + 1), cudaMemcpyDefault, s));
-        if (zb) {
-            CU(cudaMemcpyAsync(ri + nnz_off[b], lp.row_index, sizeof(int) * (size_t)zb, cudaMemcpyDefault, s));
-            CU(cudaMemcpyAsync(cv + nnz_off[b], lp.value, sizeof(double) * (size_t)zb, cudaMemcpyDefault, s));
-        }
-        if (nb) {
-            CU(cudaMemcpyAsync(obj_in + col_off[b], lp.objective, sizeof(double) * nb, cudaMemcpyDefault, s));
-            CU(cudaMemcpyAsync(lo_in + col_off[b], lp.var_lower, sizeof(double) * nb, cudaMemcpyDefault, s));
-            CU(cudaMemcpyAsync(hi_in + col_off[b], lp.var_upper, sizeof(double) * nb, cudaMemcpyDefault, s));
-        }
-        if (mb) {
-            CU(cudaMemcpyAsync(rlo_in + row_off[b], lp.row_lower, sizeof(double) * mb, cudaMemcpyDefault, s));
-            CU(cudaMemcpyAsync(rhi_in + row_off[b], lp.row_upper, sizeof(double) * mb, cudaMemcpyDefault, s));
-        }
-        if (nb > 0 && zb > 0) {  // validate in the LP's own numbering, then shift
-            ctx.begin_launch(MC_KERNEL_SETUP);
-            k_validate_csc<<<(int)((nb + kBlock - 1) / kBlock), kBlock, 0, s>>>(
-                (int)mb, (int)nb, zb, cs + col_off[b], ri + nnz_off[b], cv + nnz_off[b], counters + 2);
-            ctx.end_launch();
-        }
-        if (nb > 0) {
-            ctx.begin_launch(MC_KERNEL_SETUP);
-            kb_shift_indices<<<blocks_for(ctx, zb + nb, kBlock), kBlock, 0, s>>>(
-                cs + col_off[b], ri + nnz_off[b], (int)nb, zb, (int)nnz_off[b], (int)row_off[b]);
-            ctx.end_launch();
-        }
+        if (!lps[b].col_start) return cuda_fail(cudaErrorInvalidValue, "column pointers", __LINE__);
+        TRY(up.put(s, cs + col_off[b], lps[b].col_start, sizeof(int) * (size_t)lps[b].num_cols));
+        if (lps[b].num_cols > 0 && lps[b].nnz > 0)
+            TRY(up.put(s, ends + b, lps[b].col_start + lps[b].num_cols, sizeof(int)));
     }
-    {
-        const int total = (int)nnz;
-        CU(cudaMemcpyAsync(cs + n, &total, sizeof(int), cudaMemcpyHostToDevice, s));
+    for (int b = 0; b < count; ++b) TRY(up.put(s, ri + nnz_off[b], lps[b].row_index, sizeof(int) * (size_t)lps[b].nnz));
+    for (int b = 0; b < count; ++b) TRY(up.put(s, cv + nnz_off[b], lps[b].value, sizeof(double) * (size_t)lps[b].nnz));
+    const auto put_sides = [&](double* to, const std::vector<long long>& off, const double* mc_lp::*from,
+                               int32_t mc_lp::*size) -> int {
+        for (int b = 0; b < count; ++b) TRY(up.put(s, to + off[b], lps[b].*from, sizeof(double) * (size_t)(lps[b].*size)));
+        return MC_OK;
+    };
+    TRY(put_sides(obj_in, col_off, &mc_lp::objective, &mc_lp::num_cols));
+    TRY(put_sides(lo_in, col_off, &mc_lp::var_lower, &mc_lp::num_cols));
+    TRY(put_sides(hi_in, col_off, &mc_lp::var_upper, &mc_lp::num_cols));
+    TRY(put_sides(rlo_in, row_off, &mc_lp::row_lower, &mc_lp::num_rows));
+    TRY(put_sides(rhi_in, row_off, &mc_lp::row_upper, &mc_lp::num_rows));
+    std::vector<int> offs;
+    for (const auto* v : {&col_off, &row_off, &nnz_off}) offs.insert(offs.end(), v->begin(), v->end());
+    int* d_off = static_cast<int*>(at(o_offs));  // [3][count + 1]
+    TRY(up.put(s, d_off, offs.data(), sizeof(int) * offs.size()));
+    const int last_start = (int)nnz;
+    TRY(up.put(s, cs + n, &last_start, sizeof(int)));
+    TRY(up.flush(s));
+    if (n > 0) {
+        ctx.begin_launch(MC_KERNEL_SETUP);
+        kb_validate_csc<<<(int)((n + kBlock - 1) / kBlock), kBlock, 0, s>>>((int)n, count, d_off, d_off + count + 1,
+                                                                          d_off + 2 * (count + 1), ends, cs, ri, cv,
+                                                                          counters + 2);
+        ctx.end_launch();
+        ctx.begin_launch(MC_KERNEL_SETUP);
+        kb_shift_indices<<<blocks_for(ctx, n + nnz, kBlock), kBlock, 0, s>>>((int)n, nnz, count, d_off, d_off + count + 1,
+                                                                           d_off + 2 * (count + 1), cs, ri);
+        ctx.end_launch();
     }
     // starting points: packed like the model, a flag per LP says which parts exist
     int* warm = any_warm ? static_cast<int*>(at(o_warm)) : nullptr;
@@ -478,20 +484,22 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     for (int b = 0; b < count && any_warm; ++b) {
         if (x0 && x0[b] && lps[b].num_cols > 0) {
             warm_host[b] |= 1;
-            CU(cudaMemcpyAsync(warm_x + col_off[b], x0[b], sizeof(double) * lps[b].num_cols, cudaMemcpyDefault, s));
-        }
-        if (y0 && y0[b] && lps[b].num_rows > 0) {
-            warm_host[b] |= 2;
-            CU(cudaMemcpyAsync(warm_y + row_off[b], y0[b], sizeof(double) * lps[b].num_rows, cudaMemcpyDefault, s));
+            TRY(up.put(s, warm_x + col_off[b], x0[b], sizeof(double) * (size_t)lps[b].num_cols));
         }
     }
-    if (any_warm) CU(cudaMemcpyAsync(warm, warm_host.data(), sizeof(int) * count, cudaMemcpyHostToDevice, s));
+    for (int b = 0; b < count && any_warm; ++b)
+        if (y0 && y0[b] && lps[b].num_rows > 0) {
+            warm_host[b] |= 2;
+            TRY(up.put(s, warm_y + row_off[b], y0[b], sizeof(double) * (size_t)lps[b].num_rows));
+        }
+    if (any_warm) TRY(up.put(s, warm, warm_host.data(), sizeof(int) * (size_t)count));
     std::vector<double> host_off(2 * (size_t)count);
     for (int b = 0; b < count; ++b) {
         host_off[b] = lps[b].objective_offset;
         host_off[count + b] = lps[b].objective_sense == MC_MAXIMIZE ? -1.0 : 1.0;
     }
-    CU(cudaMemcpyAsync(offsets, host_off.data(), sizeof(double) * host_off.size(), cudaMemcpyHostToDevice, s));
+    TRY(up.put(s, offsets, host_off.data(), sizeof(double) * host_off.size()));
+    TRY(up.flush(s));
     // tile tables (lp, l0, l1 of every column tile and row tile, then each LP's
     // tile ranges), in one device buffer sized for the finest tiling
     std::vector<int> tiles_host;
@@ -734,12 +742,22 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
                                                 row_scale, stage_x, stage_y, B);
     ctx.end_launch();
     TRY(ctx.launch_check("batch unscale"));
+    // host outputs through the staging buffers (below), device outputs directly
+    std::vector<Staging::Piece> x_pieces, y_pieces;
     for (int b = 0; b < count; ++b) {
-        if (x_out && x_out[b] && lps[b].num_cols > 0)
-            CU(cudaMemcpyAsync(x_out[b], stage_x + col_off[b], sizeof(double) * lps[b].num_cols, cudaMemcpyDefault, s));
-        if (y_out && y_out[b] && lps[b].num_rows > 0)
-            CU(cudaMemcpyAsync(y_out[b], stage_y + row_off[b], sizeof(double) * lps[b].num_rows, cudaMemcpyDefault, s));
+        const bool host = lps[b].memory == MC_MEMORY_HOST;
+        const size_t xb = sizeof(double) * (size_t)lps[b].num_cols, yb = sizeof(double) * (size_t)lps[b].num_rows;
+        if (x_out && x_out[b] && xb) {
+            if (host) x_pieces.push_back({x_out[b], sizeof(double) * (size_t)col_off[b], xb});
+            else CU(cudaMemcpyAsync(x_out[b], stage_x + col_off[b], xb, cudaMemcpyDefault, s));
+        }
+        if (y_out && y_out[b] && yb) {
+            if (host) y_pieces.push_back({y_out[b], sizeof(double) * (size_t)row_off[b], yb});
+            else CU(cudaMemcpyAsync(y_out[b], stage_y + row_off[b], yb, cudaMemcpyDefault, s));
+        }
     }
+    TRY(up.get(s, stage_x, x_pieces));
+    TRY(up.get(s, stage_y, y_pieces));
     std::vector<DevState> hs(count);
     CU(cudaMemcpyAsync(hs.data(), st, sizeof(DevState) * count, cudaMemcpyDeviceToHost, s));
     std::vector<int> hcert(2 * (size_t)count);

@@ -602,13 +602,60 @@ __global__ void kb_unscale_out(const double* __restrict__ x_avg, const float* __
     }
 }
 
-// shift a packed LP's CSC indices into the packed numbering
-__global__ void kb_shift_indices(int* __restrict__ col_start, int* __restrict__ row_index, int ncols, long long nnz,
-                                 int nnz_offset, int row_offset) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nnz + ncols;
-         t += (long long)gridDim.x * blockDim.x) {
-        if (t < nnz) row_index[t] += row_offset;
-        else col_start[t - nnz] += nnz_offset;
+// The LP that item i of a packed array belongs to: off[lp] <= i < off[lp + 1].
+__device__ __forceinline__ int packed_lp(const int* __restrict__ off, int nlp, long long i) {
+    int lo = 0, hi = nlp;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (off[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// k_validate_csc for every LP of the batch, in the LPs' own numbering (before
+// kb_shift_indices); ends[lp] is the last entry of the LP's column pointers.
+__global__ void kb_validate_csc(int n, int nlp, const int* __restrict__ col_off, const int* __restrict__ row_off,
+                                const int* __restrict__ nnz_off, const int* __restrict__ ends,
+                                const int* __restrict__ col_start, const int* __restrict__ row_index,
+                                const double* __restrict__ value, int* __restrict__ bad) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const int lp = packed_lp(col_off, nlp, j);
+    const int nnz = nnz_off[lp + 1] - nnz_off[lp], m = row_off[lp + 1] - row_off[lp];
+    if (nnz == 0) return;
+    const bool last = j + 1 == col_off[lp + 1];
+    const int b = col_start[j], e = last ? ends[lp] : col_start[j + 1];
+    if (j == col_off[lp] && b != 0) atomicOr(bad, 1);
+    if (last && e != nnz) atomicOr(bad, 1);
+    if (b > e || b < 0 || e > nnz) {
+        atomicOr(bad, 1);
+        return;
+    }
+    int prev = -1;
+    for (int p = nnz_off[lp] + b; p < nnz_off[lp] + e; ++p) {
+        const int r = row_index[p];
+        const double v = value[p];
+        if (r < 0 || r >= m) { atomicOr(bad, 2); return; }
+        if (r <= prev) { atomicOr(bad, 4); return; }
+        if (!isfinite(v) || v == 0.0) { atomicOr(bad, 8); return; }
+        prev = r;
+    }
+}
+
+// Own to packed numbering: column pointers by the LP's first entry, row
+// indices by its first row.
+__global__ void kb_shift_indices(int n, long long nnz, int nlp, const int* __restrict__ col_off,
+                                 const int* __restrict__ row_off, const int* __restrict__ nnz_off,
+                                 int* __restrict__ col_start, int* __restrict__ row_index) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n + nnz;
+         i += (long long)gridDim.x * blockDim.x) {
+        if (i < n) {
+            col_start[i] += nnz_off[packed_lp(col_off, nlp, i)];
+        } else {
+            const int lp = packed_lp(nnz_off, nlp, i - n);
+            row_index[i - n] += row_off[lp];
+        }
     }
 }
 

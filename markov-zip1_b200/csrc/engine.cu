@@ -91,11 +91,127 @@ int Arena::reserve(size_t bytes) {
     return MC_OK;
 }
 
+// ---------------------------------------------------------------- staging
+void Staging::free() {
+    for (int q = 0; q < 2; ++q) {
+        if (busy[q]) cudaEventSynchronize(done[q]);
+        if (done[q]) cudaEventDestroy(done[q]);
+        done[q] = nullptr;
+        busy[q] = false;
+    }
+    if (base) cudaFreeHost(base);
+    base = nullptr;
+}
+
+int Staging::ready() {
+    if (base) return MC_OK;
+    for (cudaEvent_t& e : done)
+        if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CU(cudaMallocHost(reinterpret_cast<void**>(&base), 2 * kHalf));
+    half = 0;
+    fill = run_bytes = 0;
+    return MC_OK;
+}
+
+int Staging::turn(cudaStream_t s) {
+    TRY(flush(s));
+    CU(cudaEventRecord(done[half], s));
+    busy[half] = true;
+    half ^= 1;
+    fill = 0;
+    if (busy[half]) CU(cudaEventSynchronize(done[half]));
+    busy[half] = false;
+    return MC_OK;
+}
+
+int Staging::flush(cudaStream_t s) {
+    if (run_bytes) {
+        CU(cudaMemcpyAsync(run_dst, base + half * kHalf + run_at, run_bytes, cudaMemcpyHostToDevice, s));
+        CU(cudaEventRecord(done[half], s));
+        busy[half] = true;
+    }
+    run_bytes = 0;
+    return MC_OK;
+}
+
+// whether the host may read or write the array itself
+static bool on_host(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
+}
+
+int Staging::put(cudaStream_t s, void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return MC_OK;
+    if (!src) return cuda_fail(cudaErrorInvalidValue, "copy from NULL", __LINE__);
+    if (bytes > kHalf / 4 || !on_host(src)) {  // large arrays go as they are
+        TRY(flush(s));
+        CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s));
+        return MC_OK;
+    }
+    TRY(ready());
+    if (fill == 0 && busy[half]) {  // left by an earlier call
+        CU(cudaEventSynchronize(done[half]));
+        busy[half] = false;
+    }
+    if (fill + bytes + 16 > kHalf) TRY(turn(s));
+    if (run_bytes == 0 || static_cast<char*>(dst) != run_dst + run_bytes) {
+        TRY(flush(s));
+        run_dst = static_cast<char*>(dst);
+        run_at = fill = (fill + 15) & ~(size_t)15;
+    }
+    std::memcpy(base + half * kHalf + fill, src, bytes);
+    fill += bytes;
+    run_bytes += bytes;
+    return MC_OK;
+}
+
+int Staging::get(cudaStream_t s, const void* src, const std::vector<Piece>& pieces) {
+    if (pieces.empty()) return MC_OK;
+    TRY(ready());
+    TRY(turn(s));
+    TRY(turn(s));  // both buffers are free
+    const size_t first = pieces.front().offset, last = pieces.back().offset + pieces.back().bytes;
+    size_t next_piece = 0;
+    // the part [a, b) of the range lies in buffer q
+    auto take = [&](int q, size_t a, size_t b) {
+        while (next_piece < pieces.size()) {
+            const Piece& p = pieces[next_piece];
+            const size_t lo = std::max(a, p.offset), hi = std::min(b, p.offset + p.bytes);
+            if (lo < hi)
+                std::memcpy(static_cast<char*>(p.host) + (lo - p.offset), base + q * kHalf + (lo - a), hi - lo);
+            if (p.offset + p.bytes > b) return;
+            ++next_piece;
+        }
+    };
+    size_t before_a = 0, before_b = 0;
+    for (size_t a = first; a < last; a += kHalf) {
+        const size_t b = std::min(last, a + kHalf);
+        CU(cudaMemcpyAsync(base + half * kHalf, static_cast<const char*>(src) + a, b - a, cudaMemcpyDeviceToHost, s));
+        CU(cudaEventRecord(done[half], s));
+        if (before_b > before_a) {
+            CU(cudaEventSynchronize(done[half ^ 1]));
+            take(half ^ 1, before_a, before_b);
+        }
+        before_a = a;
+        before_b = b;
+        half ^= 1;
+    }
+    CU(cudaEventSynchronize(done[half ^ 1]));
+    take(half ^ 1, before_a, before_b);
+    fill = 0;
+    return MC_OK;
+}
+
 // ------------------------------------------------------------------ context
 Ctx::~Ctx() {
     if (device >= 0) cudaSetDevice(device);
     drop_session();
     release_graphs();
+    staging.free();
     if (arena.base) cudaFree(arena.base);
     if (h_state) cudaFreeHost(h_state);
     for (auto& e : prof_events) cudaEventDestroy(e);

@@ -66,6 +66,35 @@ struct Layout {
     }
 };
 
+// Many small copies between host and device arrays through two pinned
+// buffers of 512 KiB, used in turn: pieces that follow one another on the device
+// travel in one transfer, and the host copies into (out of) one buffer while
+// the other's transfer runs.  A copy of a pageable array of its own costs
+// 6-10 us to the device and 15-20 us back, whatever its size.
+struct Staging {
+    static constexpr size_t kHalf = 512u << 10;
+    struct Piece {
+        void* host;
+        size_t offset, bytes;  // from the start of the device range
+    };
+    char* base = nullptr;  // pinned, made at first use
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    bool busy[2] = {false, false};
+    int half = 0;
+    size_t fill = 0, run_at = 0, run_bytes = 0;
+    char* run_dst = nullptr;
+
+    void free();
+    int ready();
+    int turn(cudaStream_t s);  // to the other buffer
+    int flush(cudaStream_t s);
+    // dst (device) <- src (host or device); ends with flush()
+    int put(cudaStream_t s, void* dst, const void* src, size_t bytes);
+    // host pieces, in rising order of offset, <- device range; returns with
+    // the stream synchronised up to the copies
+    int get(cudaStream_t s, const void* src, const std::vector<Piece>& pieces);
+};
+
 struct Session;                 // a stepwise solve in progress (solve.cuh)
 void free_session(Session* s);
 
@@ -74,6 +103,7 @@ struct Ctx {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     Arena arena;
+    Staging staging;
     DevState* h_state = nullptr;  // pinned, [4]
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr;
     cudaEvent_t ev_poll[2] = {nullptr, nullptr};

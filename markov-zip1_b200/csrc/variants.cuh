@@ -1172,20 +1172,22 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     double* wx = any_wx ? static_cast<double*>(at(o_wx)) : nullptr;
     double* wy = any_wy ? static_cast<double*>(at(o_wy)) : nullptr;
     std::vector<int> hw(2 * (size_t)count, 0);
-    for (int b = 0; b < count; ++b) {
-        const double* lb = (var_lower && var_lower[b]) ? var_lower[b] : base->var_lower;
-        const double* ub = (var_upper && var_upper[b]) ? var_upper[b] : base->var_upper;
-        CU(cudaMemcpyAsync(lo_in + (size_t)b * n, lb, sizeof(double) * n, cudaMemcpyDefault, s));
-        CU(cudaMemcpyAsync(hi_in + (size_t)b * n, ub, sizeof(double) * n, cudaMemcpyDefault, s));
+    Staging& up = ctx.staging;
+    for (int b = 0; b < count; ++b)
+        TRY(up.put(s, lo_in + (size_t)b * n, (var_lower && var_lower[b]) ? var_lower[b] : base->var_lower, sizeof(double) * n));
+    for (int b = 0; b < count; ++b)
+        TRY(up.put(s, hi_in + (size_t)b * n, (var_upper && var_upper[b]) ? var_upper[b] : base->var_upper, sizeof(double) * n));
+    for (int b = 0; b < count; ++b)
         if (x0 && x0[b]) {
             hw[b] = 1;
-            CU(cudaMemcpyAsync(wx + (size_t)b * n, x0[b], sizeof(double) * n, cudaMemcpyDefault, s));
+            TRY(up.put(s, wx + (size_t)b * n, x0[b], sizeof(double) * n));
         }
+    for (int b = 0; b < count; ++b)
         if (y0 && y0[b]) {
             hw[count + b] = 1;
-            CU(cudaMemcpyAsync(wy + (size_t)b * m, y0[b], sizeof(double) * m, cudaMemcpyDefault, s));
+            TRY(up.put(s, wy + (size_t)b * m, y0[b], sizeof(double) * m));
         }
-    }
+    TRY(up.flush(s));
     CU(cudaMemcpyAsync(has_warm, hw.data(), sizeof(int) * hw.size(), cudaMemcpyHostToDevice, s));
     CU(cudaEventRecord(ctx.ev_b, s));
     int* counters = static_cast<int*>(at(o_counters));
@@ -1381,13 +1383,21 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     else kv_unscale_out<<<grid, kBlock, 0, s>>>(Bs, V, col_scale, row_scale, xo, yo);
     ctx.end_launch();
     TRY(ctx.launch_check("variant unscale"));
-    for (int k = 0; k < count; ++k) {
+    std::vector<Staging::Piece> x_pieces, y_pieces;
+    for (int k = 0; k < count; ++k) {  // slot k holds variant perm[k]
         const int b = perm[k];
-        if (x_out && x_out[b])
-            CU(cudaMemcpyAsync(x_out[b], xo + (size_t)k * n, sizeof(double) * n, cudaMemcpyDefault, s));
-        if (y_out && y_out[b])
-            CU(cudaMemcpyAsync(y_out[b], yo + (size_t)k * m, sizeof(double) * m, cudaMemcpyDefault, s));
+        const size_t xb = sizeof(double) * (size_t)n, yb = sizeof(double) * (size_t)m;
+        if (x_out && x_out[b]) {
+            if (!dev_in) x_pieces.push_back({x_out[b], (size_t)k * xb, xb});
+            else CU(cudaMemcpyAsync(x_out[b], xo + (size_t)k * n, xb, cudaMemcpyDefault, s));
+        }
+        if (y_out && y_out[b]) {
+            if (!dev_in) y_pieces.push_back({y_out[b], (size_t)k * yb, yb});
+            else CU(cudaMemcpyAsync(y_out[b], yo + (size_t)k * m, yb, cudaMemcpyDefault, s));
+        }
     }
+    TRY(up.get(s, xo, x_pieces));
+    TRY(up.get(s, yo, y_pieces));
     std::vector<DevState> hs(count + 2);
     CU(cudaMemcpyAsync(hs.data(), st, sizeof(DevState) * (count + 2), cudaMemcpyDeviceToHost, s));
     std::vector<int> hcert(2 * (size_t)count);
