@@ -7,9 +7,9 @@
 // copies block-diagonally (batch.cuh) streams the matrix K times per
 // iteration and turns every nonzero into K random 8-byte gathers.  Here the
 // iterates are stored variant-minor -- element (j, k) of an n x K array at
-// j * Kp + k, Kp = K rounded up to 32 -- and one warp carries 32 variants of
-// a line: a nonzero a_ij is loaded once per warp (a broadcast) and the
-// gathered vector entry for 32 variants is one contiguous 256-byte read.
+// j * Kp + k, Kp = K rounded up to 32 -- and neighbouring lanes carry the
+// variants of a line: a nonzero a_ij is loaded once per warp (a broadcast) and
+// the gathered vector entry for 32 variants is one contiguous read.
 //
 // Every variant still runs the reference algorithm on its own
 // (src/lp/first_order/pdlp.cpp:139-276): own step size, primal weight,
@@ -28,6 +28,8 @@
 namespace mc {
 
 constexpr int kVarWarps = kBlock / 32;  // warps per block, one line each per trip
+constexpr int kVarGathers = 4;          // gathers in flight per lane (split_dot)
+constexpr int kVarDualBlocks = 2;       // blocks per SM of the split dual kernels
 
 // The base LP (scaled, shared by every variant).
 struct VarBase {
@@ -124,9 +126,9 @@ __device__ __forceinline__ double variant_dot(const int* __restrict__ start, con
 
 // ------------------------------------------------------------------ primal
 // g = c + A^T y; x+ = clamp(x - tau g, l, u); x-bar; average; on step-size
-// iterations dx and sum col_norm dx^2 per variant (pdlp.cpp:195-206, :226)
-template <bool STEP>
-__global__ void __launch_bounds__(kBlock) kv_primal(VarBase Bs, VarRefs V, int kk) {
+// iterations dx and sum col_norm dx^2 per variant (pdlp.cpp:195-206, :226).
+// This form, with the reduction, is that of a step-size iteration.
+__global__ void __launch_bounds__(kBlock) kv_primal_step(VarBase Bs, VarRefs V, int kk) {
     __shared__ double sm[kVarWarps][33];
     MC_VARIANT_LANE(V, k, live);
     double step = 0.0, cnt = 1.0;
@@ -148,50 +150,15 @@ __global__ void __launch_bounds__(kBlock) kv_primal(VarBase Bs, VarRefs V, int k
             const double xp = clampv(__dsub_rn(xo, __dmul_rn(tau, g)), ld_stream(V.lo + q), ld_stream(V.hi + q));
             const double d = __dsub_rn(xp, xo);
             const double xbar = __dsub_rn(__dmul_rn(2.0, xp), xo);
-            if (STEP) {
-                st_keep2(V.xdx + 2 * q, xbar, d, pol);
-                acc += __dmul_rn(__dmul_rn(cn, d), d);
-            } else {
-                st_keep(V.xb + q, xbar, pol);
-            }
+            st_keep2(V.xdx + 2 * q, xbar, d, pol);
+            acc += __dmul_rn(__dmul_rn(cn, d), d);
             st_stream(V.x + q, xp);
             const double xa = ld_stream(V.xa + q);
             st_stream(V.xa + q, __dadd_rn(xa, __ddiv_rn(__dsub_rn(xp, xa), cnt)));
         }
     }
-    if (STEP) {
-        acc = lanes_reduce(acc, sm, OpSum());
-        if ((threadIdx.x >> 5) == 0 && k < V.K) var_partial(V, SLOT_DX, k)[blockIdx.x] = acc;
-    }
-}
-
-// ------------------------------------------------------------------- dual
-__device__ __forceinline__ void variant_dual_update(const VarBase& Bs, const VarRefs& V, long long i, int k,
-                                                    double ax, double sg, double cnt, unsigned long long pol) {
-    const size_t q = (size_t)i * V.Kp + k;
-    const double sigma = __ddiv_rn(sg, __ldg(Bs.row_norm + i));
-    const double v = __dadd_rn(ld_stream(V.y + q), __dmul_rn(sigma, ax));
-    const double yn =
-        __dsub_rn(v, __dmul_rn(sigma, clampv(__ddiv_rn(v, sigma), __ldg(Bs.blo + i), __ldg(Bs.bhi + i))));
-    st_keep(V.y + q, yn, pol);
-    const double ya = ld_stream(V.ya + q);
-    st_stream(V.ya + q, __dadd_rn(ya, __ddiv_rn(__dsub_rn(yn, ya), cnt)));
-}
-
-// v = y + sigma (A x-bar); y+ = v - sigma clamp(v/sigma, b_lo, b_hi); average (pdlp.cpp:220-227)
-__global__ void __launch_bounds__(kBlock) kv_dual(VarBase Bs, VarRefs V, int kk) {
-    MC_VARIANT_LANE(V, k, live);
-    double sg = 0.0, cnt = 1.0;
-    if (live) {
-        const DevState& s = V.st[k];
-        sg = s.eta * s.omega;
-        cnt = (double)(s.avg_count + kk + 1);
-    }
-    const unsigned long long pol = policy_keep();
-    MC_VARIANT_LINES(i, Bs.m) {
-        const double ax = variant_dot(Bs.rs, Bs.ci, Bs.rv, V.xb, V.Kp, i, k, live, pol);
-        if (live) variant_dual_update(Bs, V, i, k, ax, sg, cnt, pol);
-    }
+    acc = lanes_reduce(acc, sm, OpSum());
+    if ((threadIdx.x >> 5) == 0 && k < V.K) var_partial(V, SLOT_DX, k)[blockIdx.x] = acc;
 }
 
 // Step-size iteration: A x-bar (kept) and A dx from the (x-bar, dx) pairs,
@@ -254,15 +221,394 @@ __global__ void kv_step_size(VarRefs V, Controls ctl) {
     }
 }
 
-// Step-size iteration: the dual update from the kept A x-bar.
-__global__ void __launch_bounds__(kBlock) kv_dual_apply(VarBase Bs, VarRefs V, int kk) {
-    MC_VARIANT_LANE(V, k, live);
-    if (!live) return;  // no barrier follows
-    const DevState& s = V.st[k];
-    const double sg = s.eta * s.omega;
-    const double cnt = (double)(s.avg_count + kk + 1);
+// ---------------------------------------------------------- pack kernels
+// The iterations without a step-size probe reduce nothing over lines, so
+// their kernels may share the work out in another way than a warp per line
+// with one variant per lane.  That form waited: L2 was 11% busy, the issue
+// slots 42%, and a column of 8 entries was a chain of 6 dependent reads.  Two
+// forms replace it, both with the sums of variant_dot in the same order:
+//  - packs (`*_wide`): a thread carries the variants of one 16-byte load (4
+//    FP32, 2 FP64) of a line, `1 << lg` neighbouring threads (8 to 32) the
+//    whole line or a 128-byte multiple of it.  One index, one address and one
+//    gather serve the pack, the last 1-3 entries are loaded together, the
+//    line's own vectors before the gathers are waited for.
+//  - split rows (kv_dual, kvm_dual): see split_dot.
+// us per launch, before -> now, 2000 x 6000 with 8 entries a column: primal
+// (packs) FP32 18.8 -> 15.3, FP64 21.8 -> 20.1 at 128 variants, 60.5 -> 41.5 and
+// 107 -> 79 at 512 (3000 x 9000); dual 16.8 -> 14.1 and 20.3 -> 14.8 (packs, 128),
+// 12.7 -> 8.6 and 13.7 -> 10.7 (split, 32).  Columns are short, so the split
+// form gains nothing there (FP32 12.7 against 10.7 for packs at 32 variants).
+template <class T> struct PackOf;
+template <> struct PackOf<float> { using type = float4; };
+template <> struct PackOf<double> { using type = double2; };
+
+template <class T>
+struct alignas(16) Pack {
+    static constexpr int W = 16 / sizeof(T);
+    T v[W];
+};
+__device__ __forceinline__ Pack<float> ld_keep_pack(const float* a, unsigned long long pol) {
+    Pack<float> r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(a), "l"(pol));
+    return r;
+}
+__device__ __forceinline__ Pack<double> ld_keep_pack(const double* a, unsigned long long pol) {
+    Pack<double> r;
+    ld_keep2(a, pol, r.v[0], r.v[1]);
+    return r;
+}
+__device__ __forceinline__ void st_keep_pack(float* a, const Pack<float>& r, unsigned long long pol) {
+    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(a), "f"(r.v[0]), "f"(r.v[1]),
+                 "f"(r.v[2]), "f"(r.v[3]), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void st_keep_pack(double* a, const Pack<double>& r, unsigned long long pol) {
+    st_keep2(a, r.v[0], r.v[1], pol);
+}
+template <class T>
+__device__ __forceinline__ Pack<T> ld_pack(const T* a) {
+    using Q = typename PackOf<T>::type;
+    Pack<T> r;
+    *reinterpret_cast<Q*>(&r) = __ldcs(reinterpret_cast<const Q*>(a));
+    return r;
+}
+template <class T>
+__device__ __forceinline__ void st_pack(T* a, const Pack<T>& r) {
+    using Q = typename PackOf<T>::type;
+    __stcs(reinterpret_cast<Q*>(a), *reinterpret_cast<const Q*>(&r));
+}
+
+// The pack of this thread: its first variant, its lines (first, stride), and
+// per variant the step factor and averaging count of this iteration.
+template <class T>
+struct VarPack {
+    static constexpr int W = Pack<T>::W;
+    int k;
+    long long line, stride;
+    bool any, live[W];
+    T step[W], cnt[W];
+    __device__ __forceinline__ VarPack(const VarRefs& V, int lg, int kk, bool dual) {
+        k = W * ((blockIdx.y << lg) + (threadIdx.x & ((1 << lg) - 1)));
+        line = (long long)blockIdx.x * (kBlock >> lg) + (threadIdx.x >> lg);
+        stride = (long long)gridDim.x * (kBlock >> lg);
+        any = false;
+        // every state is read at once (no branch on `done` between the loads)
+        double eta[W], omega[W];
+        long long count[W];
+        int done[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const DevState& s = V.st[min(k + w, V.K - 1)];
+            done[w] = s.done;
+            eta[w] = s.eta;
+            omega[w] = s.omega;
+            count[w] = s.avg_count;
+        }
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            live[w] = k + w < V.K && !done[w];
+            any |= live[w];
+            step[w] = (T)(dual ? eta[w] * omega[w] : eta[w] / omega[w]);
+            cnt[w] = (T)(double)(count[w] + kk + 1);
+        }
+    }
+};
+
+// variant_dot for a pack: v points at the pack of line 0.  A window adds entry
+// q to sum q mod 4, the tail all of its entries to the first.
+template <int N, class T>
+__device__ __forceinline__ void pack_window(const int* __restrict__ idx, const T* __restrict__ val,
+                                            const T* __restrict__ v, int Kp, int p, unsigned long long pol,
+                                            T (&s)[4][Pack<T>::W], bool tail = false) {
+    int i[N];
+    T a[N];
+    Pack<T> g[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        i[q] = __ldg(idx + p + q);
+        a[q] = __ldg(val + p + q);
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q) g[q] = ld_keep_pack(v + (size_t)i[q] * Kp, pol);
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+#pragma unroll
+        for (int w = 0; w < Pack<T>::W; ++w) {
+            T& t = s[tail ? 0 : (q & 3)][w];
+            t = fma(a[q], g[q].v[w], t);
+        }
+}
+// AHEAD (rows): the indices of the next window are asked for before the
+// gathers of this one are waited for: dual 18.7 -> 14.1 us (128 variants, FP32).
+// Columns rarely fill one window, and the registers cost a block per SM.
+template <bool AHEAD, class T>
+__device__ __forceinline__ Pack<T> pack_dot(int b, int e, const int* __restrict__ idx, const T* __restrict__ val,
+                                            const T* __restrict__ v, int Kp, unsigned long long pol) {
+    T s[4][Pack<T>::W] = {};
+    int p = b;
+    if (!AHEAD) {
+        for (; p + 8 <= e; p += 8) pack_window<8>(idx, val, v, Kp, p, pol, s);
+    } else if (p + 8 <= e) {
+        int i[8];
+        T a[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            i[q] = __ldg(idx + p + q);
+            a[q] = __ldg(val + p + q);
+        }
+        for (; p + 8 <= e; p += 8) {
+            Pack<T> g[8];
+            T x[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                g[q] = ld_keep_pack(v + (size_t)i[q] * Kp, pol);
+                x[q] = a[q];
+            }
+            if (p + 16 <= e) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    i[q] = __ldg(idx + p + 8 + q);
+                    a[q] = __ldg(val + p + 8 + q);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int w = 0; w < Pack<T>::W; ++w) s[q & 3][w] = fma(x[q], g[q].v[w], s[q & 3][w]);
+        }
+    }
+    if (p + 4 <= e) {
+        pack_window<4>(idx, val, v, Kp, p, pol, s);
+        p += 4;
+    }
+    if (e - p == 3) pack_window<3>(idx, val, v, Kp, p, pol, s, true);
+    else if (e - p == 2) pack_window<2>(idx, val, v, Kp, p, pol, s, true);
+    else if (e - p == 1) pack_window<1>(idx, val, v, Kp, p, pol, s, true);
+    Pack<T> r;
+#pragma unroll
+    for (int w = 0; w < Pack<T>::W; ++w) r.v[w] = (s[0][w] + s[1][w]) + (s[2][w] + s[3][w]);
+    return r;
+}
+
+// Grid of a pack kernel: 1 << lg threads per line, the largest power of two up
+// to 32 that divides the packs of a line; one wave of resident blocks.
+struct WideGrid {
+    int lg;
+    dim3 grid;
+};
+template <class T, class K>
+WideGrid wide_grid(const Ctx& ctx, K kernel, long long lines, int Kp) {
+    const int packs = Kp / Pack<T>::W;
+    WideGrid g;
+    for (g.lg = 3; g.lg < 5 && packs % (2 << g.lg) == 0;) ++g.lg;
+    const int gy = packs >> g.lg;
+    const long long per_block = kBlock >> g.lg;
+    const long long wave = grid_for(ctx, kernel, 1LL << 30, 1);
+    const long long x = std::min((lines + per_block - 1) / per_block, std::max<long long>(1, wave / gy));
+    g.grid = dim3((unsigned)std::max<long long>(1, x), (unsigned)gy);
+    return g;
+}
+
+// Grid of a split dual kernel: a warp per line and 32 variants, one wave of resident blocks.
+template <class K>
+dim3 dual_grid(const Ctx& ctx, K kernel, long long lines, int groups) {
+    const long long wave = grid_for(ctx, kernel, 1LL << 30, 1);
+    const long long x = std::min((lines + kVarWarps - 1) / kVarWarps, std::max<long long>(1, wave / groups));
+    return dim3((unsigned)std::max<long long>(1, x), (unsigned)groups);
+}
+
+// From the pack of each of W neighbouring lanes, the sum over those lanes of
+// the lane's own variant (lane mod W).  FP32: (s0 + s1) + (s2 + s3).
+__device__ __forceinline__ float pack_fold(const float (&s)[1][4]) {
+    const bool b0 = threadIdx.x & 1, b1 = threadIdx.x & 2;
+    const float lo = (b0 ? s[0][1] : s[0][0]) + __shfl_xor_sync(0xffffffffu, b0 ? s[0][0] : s[0][1], 1);
+    const float hi = (b0 ? s[0][3] : s[0][2]) + __shfl_xor_sync(0xffffffffu, b0 ? s[0][2] : s[0][3], 1);
+    return (b1 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 2);
+}
+__device__ __forceinline__ double pack_fold(const double (&s)[2][2]) {
+    const bool b0 = threadIdx.x & 1;
+    const double u = (b0 ? s[0][1] : s[0][0]) + __shfl_xor_sync(0xffffffffu, b0 ? s[0][0] : s[0][1], 1);
+    const double w = (b0 ? s[1][1] : s[1][0]) + __shfl_xor_sync(0xffffffffu, b0 ? s[1][0] : s[1][1], 1);
+    return u + w;
+}
+
+// Whether a lane's pack holds a running variant.
+template <class T>
+__device__ __forceinline__ bool pack_any(bool live) {
+    constexpr int W = Pack<T>::W;
+    return (__ballot_sync(0xffffffffu, live) >> (threadIdx.x & 31 & ~(W - 1))) & ((1u << W) - 1u);
+}
+
+// variant_dot by the whole warp, for rows of many entries and few variants.
+// W neighbouring lanes share the packs of their W variants: each gathers all W
+// variants of its own one (FP64: two) of the four running sums, and pack_fold
+// hands every lane its variant.  So a warp's load covers 4 (FP64: 2) entries,
+// a row of 24 is two dependent gathers instead of six, and the next entries'
+// indices are asked for before the gathers at hand are used.  `need`: the
+// lane's pack has a running variant.
+template <class T>
+__device__ __forceinline__ T split_dot(int b, int e, const int* __restrict__ idx, const T* __restrict__ val,
+                                         const T* __restrict__ v, int Kp, int k, bool need,
+                                         unsigned long long pol) {
+    constexpr int W = Pack<T>::W, C = 4 / W, U = kVarGathers / C;  // sums per lane, windows of four per turn
+    const int q = threadIdx.x & (W - 1);
+    v += k - q;
+    const int nw = (e - b) >> 2, tail = b + 4 * nw, rest = e - tail;
+    T s[C][W] = {};
+    if (need) {
+        T ta[3];
+        Pack<T> tg[3];
+        const bool first = q == 0;
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (u < rest && first) {
+                ta[u] = __ldg(val + tail + u);
+                tg[u] = ld_keep_pack(v + (size_t)__ldg(idx + tail + u) * Kp, pol);
+            }
+        int i[U][C];
+        T a[U][C];
+        const int p = b + q;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < nw)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    i[u][c] = __ldg(idx + p + 4 * u + W * c);
+                    a[u][c] = __ldg(val + p + 4 * u + W * c);
+                }
+        for (int t = 0; t < nw; t += U) {
+            Pack<T> g[U][C];
+            T x[U][C];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t + u < nw)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        g[u][c] = ld_keep_pack(v + (size_t)i[u][c] * Kp, pol);
+                        x[u][c] = a[u][c];
+                    }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t + U + u < nw)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        i[u][c] = __ldg(idx + p + 4 * (t + U + u) + W * c);
+                        a[u][c] = __ldg(val + p + 4 * (t + U + u) + W * c);
+                    }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t + u < nw)
+#pragma unroll
+                    for (int c = 0; c < C; ++c)
+#pragma unroll
+                        for (int w = 0; w < W; ++w) s[c][w] = fma(x[u][c], g[u][c].v[w], s[c][w]);
+        }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (u < rest && first)
+#pragma unroll
+                for (int w = 0; w < W; ++w) s[0][w] = fma(ta[u], tg[u].v[w], s[0][w]);
+    }
+    return pack_fold(s);
+}
+
+// The lane's variant in a dual kernel: no reduction over lines there, so a warp
+// whose variants have all finished leaves by itself; the state is read at once.
+struct DualLane {
+    int k;
+    bool live, need;
+    double sg, cnt;
+    template <class T>
+    __device__ __forceinline__ static DualLane of(const VarRefs& V, int kk) {
+        DualLane d;
+        d.k = blockIdx.y * 32 + (threadIdx.x & 31);
+        const DevState& s = V.st[min(d.k, V.K - 1)];
+        d.live = d.k < V.K && !s.done;
+        d.sg = s.eta * s.omega;
+        d.cnt = (double)(s.avg_count + kk + 1);
+        d.need = pack_any<T>(d.live);
+        return d;
+    }
+};
+
+// the primal step of an iteration without a probe (kv_primal_step has the formulas)
+__global__ void __launch_bounds__(kBlock) kv_primal_wide(VarBase Bs, VarRefs V, int lg, int kk) {
+    const VarPack<double> me(V, lg, kk, false);
+    if (!me.any) return;
+    constexpr int W = Pack<double>::W;
     const unsigned long long pol = policy_keep();
-    MC_VARIANT_LINES(i, Bs.m) variant_dual_update(Bs, V, i, k, V.axb[(size_t)i * V.Kp + k], sg, cnt, pol);
+    for (long long j = me.line; j < Bs.n; j += me.stride) {
+        const size_t q = (size_t)j * V.Kp + me.k;
+        const int b = __ldg(Bs.cs + j), e = __ldg(Bs.cs + j + 1);
+        const double cn = __ldg(Bs.col_norm + j), cj = __ldg(Bs.c + j);
+        Pack<double> x = ld_pack(V.x + q), xa = ld_pack(V.xa + q);
+        const Pack<double> lo = ld_pack(V.lo + q), hi = ld_pack(V.hi + q);
+        Pack<double> xb = pack_dot<false>(b, e, Bs.ri, Bs.cv, V.y + me.k, V.Kp, pol);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const double g = __dadd_rn(cj, xb.v[w]);
+            const double tau = __ddiv_rn(me.step[w], cn);
+            const double xp = clampv(__dsub_rn(x.v[w], __dmul_rn(tau, g)), lo.v[w], hi.v[w]);
+            const double av = __dadd_rn(xa.v[w], __ddiv_rn(__dsub_rn(xp, xa.v[w]), me.cnt[w]));
+            xb.v[w] = __dsub_rn(__dmul_rn(2.0, xp), x.v[w]);  // a finished variant's is not read
+            x.v[w] = me.live[w] ? xp : x.v[w];
+            xa.v[w] = me.live[w] ? av : xa.v[w];
+        }
+        st_keep_pack(V.xb + q, xb, pol);
+        st_pack(V.x + q, x);
+        st_pack(V.xa + q, xa);
+    }
+}
+
+// v = y + sigma (A x-bar); y+ = v - sigma clamp(v/sigma, b_lo, b_hi); average
+// (pdlp.cpp:220-227).  With APPLY A x-bar is the kept one of a probe iteration.
+template <bool APPLY>
+__global__ void __launch_bounds__(kBlock, kVarDualBlocks) kv_dual(VarBase Bs, VarRefs V, int kk) {
+    const DualLane me = DualLane::of<double>(V, kk);
+    if (!__any_sync(0xffffffffu, me.live)) return;
+    const unsigned long long pol = policy_keep();
+    MC_VARIANT_LINES(i, Bs.m) {
+        const size_t q = (size_t)i * V.Kp + me.k;
+        const double rn = __ldg(Bs.row_norm + i), bl = __ldg(Bs.blo + i), bh = __ldg(Bs.bhi + i);
+        const double y = ld_stream(V.y + q), ya = ld_stream(V.ya + q);  // padding and finished variants included
+        const double ax = APPLY ? ld_stream(V.axb + q)
+                                : split_dot(__ldg(Bs.rs + i), __ldg(Bs.rs + i + 1), Bs.ci, Bs.rv, V.xb, V.Kp, me.k,
+                                            me.need, pol);
+        if (!me.live) continue;
+        const double sigma = __ddiv_rn(me.sg, rn);
+        const double v = __dadd_rn(y, __dmul_rn(sigma, ax));
+        const double yn = __dsub_rn(v, __dmul_rn(sigma, clampv(__ddiv_rn(v, sigma), bl, bh)));
+        st_keep(V.y + q, yn, pol);
+        st_stream(V.ya + q, __dadd_rn(ya, __ddiv_rn(__dsub_rn(yn, ya), me.cnt)));
+    }
+}
+
+// kv_dual for packs; with APPLY the dual update of a probe iteration, from the kept A x-bar
+template <bool APPLY>
+__global__ void __launch_bounds__(kBlock) kv_dual_wide(VarBase Bs, VarRefs V, int lg, int kk) {
+    const VarPack<double> me(V, lg, kk, true);
+    if (!me.any) return;
+    constexpr int W = Pack<double>::W;
+    const unsigned long long pol = policy_keep();
+    for (long long i = me.line; i < Bs.m; i += me.stride) {
+        const size_t q = (size_t)i * V.Kp + me.k;
+        const int b = __ldg(Bs.rs + i), e = __ldg(Bs.rs + i + 1);
+        const double rn = __ldg(Bs.row_norm + i), bl = __ldg(Bs.blo + i), bh = __ldg(Bs.bhi + i);
+        Pack<double> y = ld_pack(V.y + q), ya = ld_pack(V.ya + q);
+        const Pack<double> ax =
+            APPLY ? ld_pack(V.axb + q) : pack_dot<true>(b, e, Bs.ci, Bs.rv, V.xb + me.k, V.Kp, pol);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const double sigma = __ddiv_rn(me.step[w], rn);
+            const double v = __dadd_rn(y.v[w], __dmul_rn(sigma, ax.v[w]));
+            const double yn = __dsub_rn(v, __dmul_rn(sigma, clampv(__ddiv_rn(v, sigma), bl, bh)));
+            const double av = __dadd_rn(ya.v[w], __ddiv_rn(__dsub_rn(yn, ya.v[w]), me.cnt[w]));
+            y.v[w] = me.live[w] ? yn : y.v[w];
+            ya.v[w] = me.live[w] ? av : ya.v[w];
+        }
+        st_keep_pack(V.y + q, y, pol);
+        st_pack(V.ya + q, ya);
+    }
 }
 
 // --------------------------------------------------------------- residuals
@@ -593,14 +939,17 @@ struct EngineVariants {
     VarRefs V;
     Original O;
     dim3 grid;
+    WideGrid cols, wide;  // packs of columns, of rows
+    dim3 rows;
+    bool rows_wide;
     int shape_class(const DevState&) const { return 0; }
     void use_class(int) const {}
 
     int iteration(Ctx& ctx, int k, bool step, const Controls& ctl) const {
         cudaStream_t s = ctx.stream;
         ctx.begin_launch(MC_KERNEL_PRIMAL);
-        if (step) kv_primal<true><<<grid, kBlock, 0, s>>>(Bs, V, k);
-        else kv_primal<false><<<grid, kBlock, 0, s>>>(Bs, V, k);
+        if (step) kv_primal_step<<<grid, kBlock, 0, s>>>(Bs, V, k);
+        else kv_primal_wide<<<cols.grid, kBlock, 0, s>>>(Bs, V, cols.lg, k);
         ctx.end_launch();
         if (step) {
             ctx.begin_launch(MC_KERNEL_DUAL_STEP);
@@ -610,11 +959,13 @@ struct EngineVariants {
             kv_step_size<<<V.K, 256, 0, s>>>(V, ctl);
             ctx.end_launch();
             ctx.begin_launch(MC_KERNEL_DUAL_STEP);
-            kv_dual_apply<<<grid, kBlock, 0, s>>>(Bs, V, k);
+            if (rows_wide) kv_dual_wide<true><<<wide.grid, kBlock, 0, s>>>(Bs, V, wide.lg, k);
+            else kv_dual<true><<<rows, kBlock, 0, s>>>(Bs, V, k);
             ctx.end_launch();
         } else {
             ctx.begin_launch(MC_KERNEL_DUAL);
-            kv_dual<<<grid, kBlock, 0, s>>>(Bs, V, k);
+            if (rows_wide) kv_dual_wide<false><<<wide.grid, kBlock, 0, s>>>(Bs, V, wide.lg, k);
+            else kv_dual<false><<<rows, kBlock, 0, s>>>(Bs, V, k);
             ctx.end_launch();
         }
         return ctx.launch_check("variant iteration");
@@ -702,8 +1053,7 @@ __device__ __forceinline__ float variant_dot_f(const int* __restrict__ start, co
     return (s0 + s1) + (s2 + s3);
 }
 
-template <bool STEP>
-__global__ void __launch_bounds__(kBlock) kvm_primal(int n, VarRefs V, VarMixed M, int kk) {
+__global__ void __launch_bounds__(kBlock) kvm_primal_step(int n, VarRefs V, VarMixed M, int kk) {
     __shared__ double sm[kVarWarps][33];
     MC_VARIANT_LANE(V, k, live);
     float step = 0.f, cnt = 1.f;
@@ -725,53 +1075,15 @@ __global__ void __launch_bounds__(kBlock) kvm_primal(int n, VarRefs V, VarMixed 
             const float xp = clampv(__fsub_rn(xo, __fmul_rn(tau, g)), ld_stream(M.lo + q), ld_stream(M.hi + q));
             const float d = __fsub_rn(xp, xo);
             const float xbar = __fsub_rn(__fmul_rn(2.f, xp), xo);
-            if (STEP) {
-                st_keep2(M.xdx + 2 * q, xbar, d, pol);
-                acc += __dmul_rn(__dmul_rn((double)cn, (double)d), (double)d);
-            } else {
-                st_keep(M.xb + q, xbar, pol);
-            }
+            st_keep2(M.xdx + 2 * q, xbar, d, pol);
+            acc += __dmul_rn(__dmul_rn((double)cn, (double)d), (double)d);
             st_stream(M.x + q, xp);
             const float xa = ld_stream(M.xa + q);
             st_stream(M.xa + q, __fadd_rn(xa, __fdiv_rn(__fsub_rn(xp, xa), cnt)));
         }
     }
-    if (STEP) {
-        acc = lanes_reduce(acc, sm, OpSum());
-        if ((threadIdx.x >> 5) == 0 && k < V.K) var_partial(V, SLOT_DX, k)[blockIdx.x] = acc;
-    }
-}
-
-// the dual step on the correction (dual_update_mx of mixed.cuh, per variant)
-__device__ __forceinline__ void variant_dual_update_mx(const VarRefs& V, const VarMixed& M, long long i, int k,
-                                                       float ax, float sg, float cnt, unsigned long long pol) {
-    const size_t q = (size_t)i * V.Kp + k;
-    const float sigma = __fdiv_rn(sg, __ldg(M.row_norm + i));
-    const float dy = ld_stream(M.y + q), yb = ld_stream(M.yb + q);
-    const float rl = ld_stream(M.rlo + q), rh = ld_stream(M.rhi + q);
-    const float base = __fdiv_rn(__fadd_rn(yb, dy), sigma);
-    float dyn;
-    if (__fadd_rn(base, __fadd_rn(rl, ax)) < 0.f) dyn = __fadd_rn(dy, __fmul_rn(sigma, __fadd_rn(rl, ax)));
-    else if (__fadd_rn(base, __fadd_rn(rh, ax)) > 0.f) dyn = __fadd_rn(dy, __fmul_rn(sigma, __fadd_rn(rh, ax)));
-    else dyn = -yb;
-    st_keep(M.y + q, dyn, pol);
-    const float dya = ld_stream(M.ya + q);
-    st_stream(M.ya + q, __fadd_rn(dya, __fdiv_rn(__fsub_rn(dyn, dya), cnt)));
-}
-
-__global__ void __launch_bounds__(kBlock) kvm_dual(int m, VarRefs V, VarMixed M, int kk) {
-    MC_VARIANT_LANE(V, k, live);
-    float sg = 0.f, cnt = 1.f;
-    if (live) {
-        const DevState& s = V.st[k];
-        sg = (float)(s.eta * s.omega);
-        cnt = (float)(double)(s.avg_count + kk + 1);
-    }
-    const unsigned long long pol = policy_keep();
-    MC_VARIANT_LINES(i, m) {
-        const float ax = variant_dot_f(M.rs, M.ci, M.rv, M.xb, V.Kp, i, k, live, pol);
-        if (live) variant_dual_update_mx(V, M, i, k, ax, sg, cnt, pol);
-    }
+    acc = lanes_reduce(acc, sm, OpSum());
+    if ((threadIdx.x >> 5) == 0 && k < V.K) var_partial(V, SLOT_DX, k)[blockIdx.x] = acc;
 }
 
 __global__ void __launch_bounds__(kBlock) kvm_dual_probe(int m, VarRefs V, VarMixed M) {
@@ -813,14 +1125,119 @@ __global__ void __launch_bounds__(kBlock) kvm_dual_probe(int m, VarRefs V, VarMi
     if ((threadIdx.x >> 5) == 0 && k < V.K) var_partial(V, SLOT_ADX, k)[blockIdx.x] = acc;
 }
 
-__global__ void __launch_bounds__(kBlock) kvm_dual_apply(int m, VarRefs V, VarMixed M, int kk) {
-    MC_VARIANT_LANE(V, k, live);
-    if (!live) return;  // no barrier follows
-    const DevState& s = V.st[k];
-    const float sg = (float)(s.eta * s.omega);
-    const float cnt = (float)(double)(s.avg_count + kk + 1);
+// The FP32 divisions of a pack without branches, so that those of its four
+// variants overlap (primal 18.9 -> 15.6 us at 128 variants): a / b =
+// float(a * recip_wide(b)), correctly rounded.  For floats a, b and a rounding
+// boundary c (25 bits), |a - c b| is 0 or at least one unit of its last place,
+// so a / b differs from c by 0 or at least 2^-49 of itself, eight times the
+// error of the FP64 product; and FP64 has room for every float quotient.  (A
+// tie, |a - c b| = 0, exists only among quotients below 2^-126, where the last
+// bit may differ from the divide's.)  The reciprocal starts from the hardware's
+// approximation (about 2^-23) and takes one third-order step (e -> e^3); a b
+// whose approximation is no good (zero, tiny, huge, not finite) is divided.
+__device__ __forceinline__ double recip_wide(float b) {
+    const double y = (double)__fdividef(1.f, b), e = fma(-(double)b, y, 1.0);
+    if (!(fabs(e) < 1e-6)) return __ddiv_rn(1.0, (double)b);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ float div_wide(float a, double y) { return (float)__dmul_rn((double)a, y); }
+
+// the primal step of an iteration without a probe, on the correction
+__global__ void __launch_bounds__(kBlock) kvm_primal_wide(int n, VarRefs V, VarMixed M, int lg, int kk) {
+    const VarPack<float> me(V, lg, kk, false);
+    if (!me.any) return;
+    constexpr int W = Pack<float>::W;
+    double rcnt[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) rcnt[w] = recip_wide(me.cnt[w]);
     const unsigned long long pol = policy_keep();
-    MC_VARIANT_LINES(i, m) variant_dual_update_mx(V, M, i, k, M.axb[(size_t)i * V.Kp + k], sg, cnt, pol);
+    for (long long j = me.line; j < n; j += me.stride) {
+        const size_t q = (size_t)j * V.Kp + me.k;
+        const int b = __ldg(M.cs + j), e = __ldg(M.cs + j + 1);
+        const float cn = __ldg(M.col_norm + j);
+        Pack<float> x = ld_pack(M.x + q), xa = ld_pack(M.xa + q);
+        const Pack<float> g = ld_pack(M.g + q), lo = ld_pack(M.lo + q), hi = ld_pack(M.hi + q);
+        const double rcn = recip_wide(cn);
+        Pack<float> xb = pack_dot<false>(b, e, M.ri, M.cv, M.y + me.k, V.Kp, pol);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const float gw = __fadd_rn(g.v[w], xb.v[w]);
+            const float tau = div_wide(me.step[w], rcn);
+            const float xp = clampv(__fsub_rn(x.v[w], __fmul_rn(tau, gw)), lo.v[w], hi.v[w]);
+            const float av = __fadd_rn(xa.v[w], div_wide(__fsub_rn(xp, xa.v[w]), rcnt[w]));
+            xb.v[w] = __fsub_rn(__fmul_rn(2.f, xp), x.v[w]);  // a finished variant's is not read
+            x.v[w] = me.live[w] ? xp : x.v[w];
+            xa.v[w] = me.live[w] ? av : xa.v[w];
+        }
+        st_keep_pack(M.xb + q, xb, pol);
+        st_pack(M.x + q, x);
+        st_pack(M.xa + q, xa);
+    }
+}
+
+// the dual step on the correction (dual_update_mx of mixed.cuh, per variant)
+template <bool APPLY>
+__global__ void __launch_bounds__(kBlock, kVarDualBlocks) kvm_dual(int m, VarRefs V, VarMixed M, int kk) {
+    const DualLane me = DualLane::of<float>(V, kk);
+    if (!__any_sync(0xffffffffu, me.live)) return;
+    const float sg = (float)me.sg, cnt = (float)me.cnt;
+    const unsigned long long pol = policy_keep();
+    MC_VARIANT_LINES(i, m) {
+        const size_t q = (size_t)i * V.Kp + me.k;
+        const float rn = __ldg(M.row_norm + i);
+        const float dy = ld_stream(M.y + q), dya = ld_stream(M.ya + q), yb = ld_stream(M.yb + q);
+        const float rl = ld_stream(M.rlo + q), rh = ld_stream(M.rhi + q);
+        const float ax = APPLY ? ld_stream(M.axb + q)
+                               : split_dot(__ldg(M.rs + i), __ldg(M.rs + i + 1), M.ci, M.rv, M.xb, V.Kp, me.k,
+                                           me.need, pol);
+        if (!me.live) continue;
+        const float sigma = __fdiv_rn(sg, rn);
+        const float base = __fdiv_rn(__fadd_rn(yb, dy), sigma);
+        const float tl = __fadd_rn(rl, ax), th = __fadd_rn(rh, ax);
+        const bool below = __fadd_rn(base, tl) < 0.f, above = __fadd_rn(base, th) > 0.f;
+        const float moved = __fadd_rn(dy, __fmul_rn(sigma, below ? tl : th));
+        const float dyn = (below || above) ? moved : -yb;
+        st_keep(M.y + q, dyn, pol);
+        st_stream(M.ya + q, __fadd_rn(dya, __fdiv_rn(__fsub_rn(dyn, dya), cnt)));
+    }
+}
+
+// kvm_dual for packs; with APPLY the dual update of a probe iteration, from the kept A dx-bar
+template <bool APPLY>
+__global__ void __launch_bounds__(kBlock) kvm_dual_wide(int m, VarRefs V, VarMixed M, int lg, int kk) {
+    const VarPack<float> me(V, lg, kk, true);
+    if (!me.any) return;
+    constexpr int W = Pack<float>::W;
+    double rcnt[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) rcnt[w] = recip_wide(me.cnt[w]);
+    const unsigned long long pol = policy_keep();
+    for (long long i = me.line; i < m; i += me.stride) {
+        const size_t q = (size_t)i * V.Kp + me.k;
+        const int b = __ldg(M.rs + i), e = __ldg(M.rs + i + 1);
+        const float rn = __ldg(M.row_norm + i);
+        Pack<float> y = ld_pack(M.y + q), ya = ld_pack(M.ya + q);
+        const Pack<float> yb = ld_pack(M.yb + q), rl = ld_pack(M.rlo + q), rh = ld_pack(M.rhi + q);
+        const double rrn = recip_wide(rn);
+        const Pack<float> ax =
+            APPLY ? ld_pack(M.axb + q) : pack_dot<true>(b, e, M.ci, M.rv, M.xb + me.k, V.Kp, pol);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            // the dual step on the correction (dual_update_mx of mixed.cuh)
+            const float dy = y.v[w];
+            const float sigma = div_wide(me.step[w], rrn);
+            const float base = div_wide(__fadd_rn(yb.v[w], dy), recip_wide(sigma));
+            const float tl = __fadd_rn(rl.v[w], ax.v[w]), th = __fadd_rn(rh.v[w], ax.v[w]);
+            const bool below = __fadd_rn(base, tl) < 0.f, above = __fadd_rn(base, th) > 0.f;
+            const float moved = __fadd_rn(dy, __fmul_rn(sigma, below ? tl : th));
+            const float dyn = (below || above) ? moved : -yb.v[w];
+            const float av = __fadd_rn(ya.v[w], div_wide(__fsub_rn(dyn, ya.v[w]), rcnt[w]));
+            y.v[w] = me.live[w] ? dyn : dy;
+            ya.v[w] = me.live[w] ? av : ya.v[w];
+        }
+        st_keep_pack(M.y + q, y, pol);
+        st_pack(M.ya + q, ya);
+    }
 }
 
 // FP64 residual pass on xh + dx_avg, yh + dy_avg (FP64 matrix of the base),
@@ -967,14 +1384,17 @@ struct EngineVariantsMixed {
     VarMixed M;
     Original O;
     dim3 grid;
+    WideGrid cols, wide;  // packs of columns, of rows
+    dim3 rows;
+    bool rows_wide;
     int shape_class(const DevState&) const { return 0; }
     void use_class(int) const {}
 
     int iteration(Ctx& ctx, int k, bool step, const Controls& ctl) const {
         cudaStream_t s = ctx.stream;
         ctx.begin_launch(MC_KERNEL_PRIMAL);
-        if (step) kvm_primal<true><<<grid, kBlock, 0, s>>>(Bs.n, V, M, k);
-        else kvm_primal<false><<<grid, kBlock, 0, s>>>(Bs.n, V, M, k);
+        if (step) kvm_primal_step<<<grid, kBlock, 0, s>>>(Bs.n, V, M, k);
+        else kvm_primal_wide<<<cols.grid, kBlock, 0, s>>>(Bs.n, V, M, cols.lg, k);
         ctx.end_launch();
         if (step) {
             ctx.begin_launch(MC_KERNEL_DUAL_STEP);
@@ -984,11 +1404,13 @@ struct EngineVariantsMixed {
             kv_step_size<<<V.K, 256, 0, s>>>(V, ctl);
             ctx.end_launch();
             ctx.begin_launch(MC_KERNEL_DUAL_STEP);
-            kvm_dual_apply<<<grid, kBlock, 0, s>>>(Bs.m, V, M, k);
+            if (rows_wide) kvm_dual_wide<true><<<wide.grid, kBlock, 0, s>>>(Bs.m, V, M, wide.lg, k);
+            else kvm_dual<true><<<rows, kBlock, 0, s>>>(Bs.m, V, M, k);
             ctx.end_launch();
         } else {
             ctx.begin_launch(MC_KERNEL_DUAL);
-            kvm_dual<<<grid, kBlock, 0, s>>>(Bs.m, V, M, k);
+            if (rows_wide) kvm_dual_wide<false><<<wide.grid, kBlock, 0, s>>>(Bs.m, V, M, wide.lg, k);
+            else kvm_dual<false><<<rows, kBlock, 0, s>>>(Bs.m, V, M, k);
             ctx.end_launch();
         }
         return ctx.launch_check("variant iteration (FP32)");
@@ -1301,12 +1723,22 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     TraceBuf tr{0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     const int poll_every = o->check_every_chunks > 0 ? o->check_every_chunks : 1;
     VarMixed M{};
+    // Rows go to the split form while one wave of its warps takes them all,
+    // else to packs, which issue fewer instructions: us per dual launch split /
+    // packs / one variant per lane, 8 entries a column: 8.6 / 17.2 / 12.7 (32 x
+    // 2000 rows, FP32), 10.6 / 12.6 / 13.7 (FP64); 18.1 / 14.1 / 16.8 (128 x 2000,
+    // FP32), 20.9 / 14.8 / 20.3 (FP64).
+    const bool rows_wide = (long long)m * groups > (long long)ctx.sm_count * kVarDualBlocks * kVarWarps;
     if (!mixed) {
         EngineVariants eng;
         eng.Bs = Bs;
         eng.V = V;
         eng.O = O;
         eng.grid = grid;
+        eng.cols = wide_grid<double>(ctx, kv_primal_wide, n, Kp);
+        eng.rows = dual_grid(ctx, kv_dual<false>, m, groups);
+        eng.wide = wide_grid<double>(ctx, kv_dual_wide<false>, m, Kp);
+        eng.rows_wide = rows_wide;
         TRY(run_chunks(ctx, eng, V.global, o->max_iterations, o->restart_every, poll_every, ctl, tr));
     } else {
         float* f_cv = static_cast<float*>(at(o_f_cv));
@@ -1368,6 +1800,10 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
         eng.M = M;
         eng.O = O;
         eng.grid = grid;
+        eng.cols = wide_grid<float>(ctx, kvm_primal_wide, n, Kp);
+        eng.rows = dual_grid(ctx, kvm_dual<false>, m, groups);
+        eng.wide = wide_grid<float>(ctx, kvm_dual_wide<false>, m, Kp);
+        eng.rows_wide = rows_wide;
         // the first correction LP of every running variant, around its start
         TRY(eng.residual_pass(ctx));
         TRY(eng.recenter(ctx, 1));
