@@ -87,149 +87,293 @@ struct Layout {
 // ----------------------------------------------------------------- kernels
 // Y[N x H] = act(X1[N x K1] W1[K1 x H] + X2[N x K2] W2[K2 x H] + b)
 //
-// Tiled: a block computes a 64-row tile of Y; the weights (K x 64) and the
-// tile's input rows are staged in shared memory once, and each of the 256
-// threads accumulates a 4 x 4 register block (rows ty*4.., columns tx*4..),
-// so every weight and input value is read from global memory once per tile
-// instead of once per output.  Each output sums b, then X1 W1 over k in
-// order, then X2 W2 -- the order of the one-thread-per-output form.
+// Tiled: a block computes a TR-row tile of Y; the weights (K x 64) and the
+// tile's input rows are staged in shared memory, and each of the 256 threads
+// accumulates a TR/16 x 4 register block, so every weight and input value is
+// read from global memory once per tile.  Each output sums b, then X1 W1 over
+// k in order, then X2 W2.  At the sizes of a training instance (thousands of
+// rows) a block waits for its loads, not for arithmetic: both parts' inputs
+// and weights are asked for at once, 16 bytes a load, and tiles of 32 rows
+// keep two blocks on an SM (9001 rows: 27.5 -> 8.6 us); with more tiles than
+// that, 64 rows halve the weight traffic.
 constexpr int kTile = 64;
-__device__ __forceinline__ void dense_stage(float (*sA)[kTile + 1], float (*sW)[H], const float* __restrict__ A,
-                                            int K, const float* __restrict__ W, long long r0, int rows) {
-    for (int q = threadIdx.x; q < kTile * kTile; q += blockDim.x) {
-        const int rr = q / kTile, kk = q % kTile;
-        sA[rr][kk] = (rr < rows && kk < K) ? A[(r0 + rr) * K + kk] : 0.f;
-    }
-    for (int q = threadIdx.x; q < K * H; q += blockDim.x) sW[q / H][q % H] = W[q];
+constexpr int kPad = kTile + 4;  // row stride in shared memory: 16-byte rows, spread over the banks
+
+__device__ __forceinline__ float4 ld4(const float* a, bool in) {
+    return in ? *reinterpret_cast<const float4*>(a) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// the 16-byte piece u of this thread of a tile of ROWS x 64: row, column
+__device__ __forceinline__ int tile_row(int u) { return (threadIdx.x + kThreads * u) / 16; }
+__device__ __forceinline__ int tile_col() { return threadIdx.x % 16 * 4; }
+
+// dZ = dY where not Y <= 0
+__device__ __forceinline__ float4 relu_bwd(float4 y, float4 z) {
+    if (y.x <= 0.f) z.x = 0.f;
+    if (y.y <= 0.f) z.y = 0.f;
+    if (y.z <= 0.f) z.z = 0.f;
+    if (y.w <= 0.f) z.w = 0.f;
+    return z;
 }
 
+template <int TR>
 __global__ void __launch_bounds__(kThreads) g_dense_fwd(int N, const float* __restrict__ X1, int K1,
                                                         const float* __restrict__ W1, const float* __restrict__ X2,
-                                                        int K2, const float* __restrict__ W2,
-                                                        const float* __restrict__ b, float* __restrict__ Y, int relu) {
-    __shared__ float sA[kTile][kTile + 1];
+                                                        const float* __restrict__ W2, const float* __restrict__ b,
+                                                        float* __restrict__ Y) {
+    __shared__ __align__(16) float sA[TR][kPad];
     __shared__ __align__(16) float sW[kTile][H];
+    constexpr int RI = TR / 16;
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    for (long long r0 = (long long)blockIdx.x * kTile; r0 < N; r0 += (long long)gridDim.x * kTile) {
-        const int rows = (int)(N - r0 < kTile ? N - r0 : kTile);
-        float acc[4][4];
+    for (long long r0 = (long long)blockIdx.x * TR; r0 < N; r0 += (long long)gridDim.x * TR) {
+        const int rows = (int)(N - r0 < TR ? N - r0 : TR);
+        float acc[RI][4];
         for (int j = 0; j < 4; ++j) {
             const float bj = b[tx * 4 + j];
-            for (int i = 0; i < 4; ++i) acc[i][j] = bj;
+            for (int i = 0; i < RI; ++i) acc[i][j] = bj;
         }
-        for (int part = 0; part < 2; ++part) {
-            const float* X = part ? X2 : X1;
-            const float* W = part ? W2 : W1;
-            const int K = part ? K2 : K1;
-            if (!X) continue;
-            __syncthreads();
-            dense_stage(sA, sW, X, K, W, r0, rows);
-            __syncthreads();
-            for (int k = 0; k < K; ++k) {
-                const float4 w = *reinterpret_cast<const float4*>(&sW[k][tx * 4]);
-                for (int i = 0; i < 4; ++i) {
-                    const float x = sA[ty * 4 + i][k];
-                    acc[i][0] = fmaf(x, w.x, acc[i][0]);
-                    acc[i][1] = fmaf(x, w.y, acc[i][1]);
-                    acc[i][2] = fmaf(x, w.z, acc[i][2]);
-                    acc[i][3] = fmaf(x, w.w, acc[i][3]);
+        auto add = [&](int k, const float (&x)[RI]) {
+            const float4 w = *reinterpret_cast<const float4*>(&sW[k][tx * 4]);
+            for (int i = 0; i < RI; ++i) {
+                acc[i][0] = fmaf(x[i], w.x, acc[i][0]);
+                acc[i][1] = fmaf(x[i], w.y, acc[i][1]);
+                acc[i][2] = fmaf(x[i], w.z, acc[i][2]);
+                acc[i][3] = fmaf(x[i], w.w, acc[i][3]);
+            }
+        };
+        if (X2) {  // both H wide
+            float4 va[2][RI], vw[2][4];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                const float* X = part ? X2 : X1;
+                const float* W = part ? W2 : W1;
+#pragma unroll
+                for (int u = 0; u < RI; ++u)
+                    va[part][u] = ld4(X + (r0 + tile_row(u)) * H + tile_col(), tile_row(u) < rows);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) vw[part][u] = ld4(W + tile_row(u) * H + tile_col(), true);
+            }
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < RI; ++u)
+                    *reinterpret_cast<float4*>(&sA[tile_row(u)][tile_col()]) = va[part][u];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(&sW[tile_row(u)][tile_col()]) = vw[part][u];
+                __syncthreads();
+#pragma unroll 4
+                for (int k = 0; k < H; k += 4) {
+                    float4 x4[RI];
+                    for (int i = 0; i < RI; ++i) x4[i] = *reinterpret_cast<const float4*>(&sA[ty * RI + i][k]);
+                    float x[RI];
+                    for (int i = 0; i < RI; ++i) x[i] = x4[i].x;
+                    add(k, x);
+                    for (int i = 0; i < RI; ++i) x[i] = x4[i].y;
+                    add(k + 1, x);
+                    for (int i = 0; i < RI; ++i) x[i] = x4[i].z;
+                    add(k + 2, x);
+                    for (int i = 0; i < RI; ++i) x[i] = x4[i].w;
+                    add(k + 3, x);
                 }
             }
-        }
-        for (int i = 0; i < 4; ++i) {
-            const int rr = ty * 4 + i;
-            if (rr >= rows) continue;
-            float* y = Y + (r0 + rr) * H + tx * 4;
-            for (int j = 0; j < 4; ++j) y[j] = relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
-        }
-    }
-}
-
-// dZ = dY * (Y > 0) in place (relu backward)
-__global__ void g_relu_bwd(long long count, const float* __restrict__ Y, float* __restrict__ dY) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < count;
-         t += (long long)gridDim.x * blockDim.x)
-        if (Y[t] <= 0.f) dY[t] = 0.f;
-}
-
-// dX[N x K] (+)= dZ[N x H] W[K x H]^T
-//
-// Tiled like g_dense_fwd: a 64-row tile of dZ and all of W in shared memory,
-// a 4 x 4 register block per thread (rows ty*4.., output columns tx*4..);
-// each output sums over c = 0..H-1 in order, as the one-thread-per-output form.
-__global__ void __launch_bounds__(kThreads) g_dense_bwd_x(int N, const float* __restrict__ dZ,
-                                                          const float* __restrict__ W, int K, float* __restrict__ dX,
-                                                          int accumulate) {
-    __shared__ float sZ[kTile][H + 1];
-    __shared__ float sW[kTile][H + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    for (int q = threadIdx.x; q < K * H; q += blockDim.x) sW[q / H][q % H] = W[q];
-    for (long long r0 = (long long)blockIdx.x * kTile; r0 < N; r0 += (long long)gridDim.x * kTile) {
-        const int rows = (int)(N - r0 < kTile ? N - r0 : kTile);
-        __syncthreads();
-        for (int q = threadIdx.x; q < kTile * H; q += blockDim.x) {
-            const int rr = q / H, cc = q % H;
-            sZ[rr][cc] = (rr < rows) ? dZ[(r0 + rr) * H + cc] : 0.f;
-        }
-        __syncthreads();
-        float acc[4][4] = {};
-        for (int c = 0; c < H; ++c) {
-            float w[4], z[4];
-            for (int j = 0; j < 4; ++j) w[j] = (tx * 4 + j < K) ? sW[tx * 4 + j][c] : 0.f;
-            for (int i = 0; i < 4; ++i) z[i] = sZ[ty * 4 + i][c];
-            for (int i = 0; i < 4; ++i)
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(z[i], w[j], acc[i][j]);
-        }
-        for (int i = 0; i < 4; ++i) {
-            const int rr = ty * 4 + i;
-            if (rr >= rows) continue;
-            for (int j = 0; j < 4; ++j) {
-                const int k = tx * 4 + j;
-                if (k >= K) continue;
-                float* d = dX + (r0 + rr) * K + k;
-                *d = accumulate ? *d + acc[i][j] : acc[i][j];
+        } else {  // the encoders: a few features
+            __syncthreads();
+            for (int q = threadIdx.x; q < rows * K1; q += blockDim.x) sA[q / K1][q % K1] = X1[r0 * K1 + q];
+            for (int q = threadIdx.x; q < K1 * H; q += blockDim.x) sW[q / H][q % H] = W1[q];
+            __syncthreads();
+            for (int k = 0; k < K1; ++k) {
+                float x[RI];
+                for (int i = 0; i < RI; ++i) x[i] = ty * RI + i < rows ? sA[ty * RI + i][k] : 0.f;
+                add(k, x);
             }
         }
+        for (int i = 0; i < RI; ++i) {
+            const int rr = ty * RI + i;
+            if (rr >= rows) continue;
+            *reinterpret_cast<float4*>(Y + (r0 + rr) * H + tx * 4) =
+                make_float4(fmaxf(acc[i][0], 0.f), fmaxf(acc[i][1], 0.f), fmaxf(acc[i][2], 0.f), fmaxf(acc[i][3], 0.f));
+        }
     }
 }
 
+// Backward of Y = relu(X1 W1 + X2 W2 + b) for a tile of kRows rows, dZ = dY
+// where not Y <= 0:
+//   dX1 = dZ W1^T, dX2 = dZ W2^T             (each output over c in order)
+//   block partials of X1^T dZ, X2^T dZ and of the column sums of dZ (over the
+//   tile's rows in order): part holds [blocks x H x H] twice, then [blocks x H].
+// One launch instead of six (mask, two weight gradients, two products, each
+// reading dZ again: 5 to 16 us each at 9001 rows; now 14.5).  A block is 64 x 64 x 64 four
+// times: a thread accumulates 4 x 4 outputs from 16-byte shared loads, and the
+// second operands are on their way while the first are used.
+__global__ void __launch_bounds__(kThreads) g_update_bwd(int N, const float* __restrict__ Y,
+                                                         const float* __restrict__ dY, const float* __restrict__ X1,
+                                                         const float* __restrict__ X2, const float* __restrict__ W1,
+                                                         const float* __restrict__ W2, float* __restrict__ dX1,
+                                                         float* __restrict__ dX2, float* __restrict__ part) {
+    extern __shared__ __align__(16) float smem[];
+    auto sZ = reinterpret_cast<float(*)[kPad]>(smem);
+    auto sX = sZ + kRows;
+    auto sW = sX + kRows;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const long long r0 = (long long)blockIdx.x * kRows;
+    const int rows = (int)(N - r0 < kRows ? N - r0 : kRows);
+    float4 vx[4], vw[4];
+    {
+        float4 vy[4], vz[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool in = tile_row(u) < rows;
+            const long long q = (r0 + tile_row(u)) * H + tile_col();
+            vy[u] = ld4(Y + q, in);
+            vz[u] = ld4(dY + q, in);
+            vx[u] = ld4(X1 + q, in);
+            vw[u] = ld4(W1 + tile_row(u) * H + tile_col(), true);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            *reinterpret_cast<float4*>(&sZ[tile_row(u)][tile_col()]) = relu_bwd(vy[u], vz[u]);
+        }
+    }
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+        if (side) __syncthreads();  // the first operands are used up
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            *reinterpret_cast<float4*>(&sX[tile_row(u)][tile_col()]) = vx[u];
+            *reinterpret_cast<float4*>(&sW[tile_row(u)][tile_col()]) = vw[u];
+        }
+        __syncthreads();
+        if (!side) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                vx[u] = ld4(X2 + (r0 + tile_row(u)) * H + tile_col(), tile_row(u) < rows);
+                vw[u] = ld4(W2 + tile_row(u) * H + tile_col(), true);
+            }
+        }
+        {  // rows ty*4 + i, columns tx + 16 j (rows of sW 16 apart: no bank conflict)
+            float acc[4][4] = {};
+#pragma unroll 4
+            for (int c = 0; c < H; c += 4) {
+                float4 z[4], w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) z[i] = *reinterpret_cast<const float4*>(&sZ[ty * 4 + i][c]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(&sW[tx + 16 * j][c]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float t = fmaf(z[i].x, w[j].x, acc[i][j]);
+                        t = fmaf(z[i].y, w[j].y, t);
+                        t = fmaf(z[i].z, w[j].z, t);
+                        acc[i][j] = fmaf(z[i].w, w[j].w, t);
+                    }
+            }
+            float* dX = side ? dX2 : dX1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (ty * 4 + i < rows)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) dX[(r0 + ty * 4 + i) * H + tx + 16 * j] = acc[i][j];
+        }
+        {  // rows k = ty*4 + i, columns tx*4 + j of the weight gradient
+            float acc[4][4] = {};
+#pragma unroll 4
+            for (int rr = 0; rr < rows; ++rr) {
+                const float4 x = *reinterpret_cast<const float4*>(&sX[rr][ty * 4]);
+                const float4 z = *reinterpret_cast<const float4*>(&sZ[rr][tx * 4]);
+                const float xs[4] = {x.x, x.y, x.z, x.w}, zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], zs[j], acc[i][j]);
+            }
+            float* pw = part + ((long long)side * gridDim.x + blockIdx.x) * H * H;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(pw + (ty * 4 + i) * H + tx * 4) =
+                    make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+    }
+    if (threadIdx.x < H) {
+        float acc = 0.f;
+#pragma unroll 8
+        for (int rr = 0; rr < rows; ++rr) acc += sZ[rr][threadIdx.x];
+        part[2LL * gridDim.x * H * H + (long long)blockIdx.x * H + threadIdx.x] = acc;
+    }
+}
+constexpr int kUpdateSmem = 3 * kRows * kPad * (int)sizeof(float);
+
 // block partials of X^T dZ ([K x H]) and of the column sums of dZ ([H]) over
-// kRows rows per block
+// kRows rows per block, dZ = dY where not Y <= 0 (the encoders: K features)
 __global__ void __launch_bounds__(kThreads) g_dense_bwd_w(int N, const float* __restrict__ X, int K,
-                                                          const float* __restrict__ dZ,
+                                                          const float* __restrict__ Y,
+                                                          const float* __restrict__ dY,
                                                           float* __restrict__ part_w, float* __restrict__ part_b) {
-    __shared__ float sx[kRows * H];
-    __shared__ float sz[kRows * H];
+    __shared__ float sx[kRows * FV];
+    __shared__ __align__(16) float sz[kRows * H];
     const int r0 = blockIdx.x * kRows;
     const int rows = min(kRows, N - r0);
-    for (int q = threadIdx.x; q < kRows * H; q += blockDim.x) {
-        const int rr = q / H, cc = q % H;
-        sz[q] = (rr < rows) ? dZ[(long long)(r0 + rr) * H + cc] : 0.f;
-        sx[q] = (rr < rows && cc < K) ? X[(long long)(r0 + rr) * K + cc] : 0.f;
+    float4 vy[4], vz[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const long long at = (long long)(r0 + tile_row(u)) * H + tile_col();
+        vy[u] = ld4(Y + at, tile_row(u) < rows);
+        vz[u] = ld4(dY + at, tile_row(u) < rows);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(&sz[tile_row(u) * H + tile_col()]) = relu_bwd(vy[u], vz[u]);
+    for (int q = threadIdx.x; q < rows * K; q += kThreads) sx[q] = X[(long long)r0 * K + q];
     __syncthreads();
     float* pw = part_w + (long long)blockIdx.x * K * H;
     for (int q = threadIdx.x; q < K * H; q += blockDim.x) {
         const int k = q / H, c = q % H;
         float acc = 0.f;
-        for (int rr = 0; rr < rows; ++rr) acc = fmaf(sx[rr * H + k], sz[rr * H + c], acc);
+#pragma unroll 8
+        for (int rr = 0; rr < rows; ++rr) acc = fmaf(sx[rr * K + k], sz[rr * H + c], acc);
         pw[q] = acc;
     }
-    if (part_b)
-        for (int c = threadIdx.x; c < H; c += blockDim.x) {
-            float acc = 0.f;
-            for (int rr = 0; rr < rows; ++rr) acc += sz[rr * H + c];
-            part_b[(long long)blockIdx.x * H + c] = acc;
-        }
+    for (int c = threadIdx.x; c < H; c += blockDim.x) {
+        float acc = 0.f;
+        for (int rr = 0; rr < rows; ++rr) acc += sz[rr * H + c];
+        part_b[(long long)blockIdx.x * H + c] = acc;
+    }
 }
 
-// out[q] += sum over blocks of part[b][q], in block order
-__global__ void g_reduce_parts(int blocks, int width, const float* __restrict__ part, float* __restrict__ out) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < width; q += gridDim.x * blockDim.x) {
-        float acc = 0.f;
-        for (int b = 0; b < blocks; ++b) acc += part[(long long)b * width + q];
-        out[q] += acc;
+// out[q] += sum over blocks of part[b][q], in block order, for up to three
+// arrays.  A thread's sum is a chain of loads: 32 are in flight at a time, and
+// the arrays of one update share a launch (141 blocks, from DRAM: three
+// launches of 10-13 us -> one of 10).
+struct Parts {
+    const float* part;  // [blocks x width]
+    float* out;
+    int width;
+};
+constexpr int kReduceThreads = 64;
+__global__ void __launch_bounds__(kReduceThreads) g_reduce_parts(int blocks, Parts a, Parts b, Parts c) {
+    int q = blockIdx.x * kReduceThreads + threadIdx.x;
+    if (q >= a.width) {
+        q -= a.width;
+        a = b;
+        if (q >= a.width) {
+            q -= a.width;
+            a = c;
+            if (q >= a.width) return;
+        }
     }
+    float acc = 0.f;
+    const float* p = a.part + q;
+    int i = 0;
+    for (; i + 32 <= blocks; i += 32) {
+        float v[32];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) v[u] = p[(long long)(i + u) * a.width];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) acc += v[u];
+    }
+#pragma unroll 8
+    for (; i < blocks; ++i) acc += p[(long long)i * a.width];
+    a.out[q] += acc;
 }
 
 // Out[line][:] (+)= sum_p val[p] * s_line[line] * s_idx[idx[p]] * In[idx[p]][:]
@@ -243,11 +387,29 @@ __global__ void g_aggregate(int lines, const int* __restrict__ start, const int*
          w += ((long long)gridDim.x * blockDim.x) >> 5) {
         float a0 = 0.f, a1 = 0.f;
         const float sl = s_line ? s_line[w] : 1.f;
-        for (int p = start[w]; p < start[w + 1]; ++p) {
-            const int j = idx[p];
-            const float wgt = val[p] * sl * (s_idx ? s_idx[j] : 1.f);
-            a0 = fmaf(wgt, In[(long long)j * H + lane], a0);
-            a1 = fmaf(wgt, In[(long long)j * H + 32 + lane], a1);
+        const int e = start[w + 1];
+        for (int p = start[w]; p < e; p += 4) {  // four entries in flight, added in order
+            int j[4];
+            float v[4], x0[4], x1[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (p + u < e) {
+                    j[u] = idx[p + u];
+                    v[u] = val[p + u];
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (p + u < e) {
+                    v[u] = v[u] * sl * (s_idx ? s_idx[j[u]] : 1.f);
+                    x0[u] = In[(long long)j[u] * H + lane];
+                    x1[u] = In[(long long)j[u] * H + 32 + lane];
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (p + u < e) {
+                    a0 = fmaf(v[u], x0[u], a0);
+                    a1 = fmaf(v[u], x1[u], a1);
+                }
         }
         float* o = Out + w * H;
         if (accumulate) {
@@ -265,7 +427,14 @@ __global__ void g_readout(int N, const float* __restrict__ X, const float* __res
                           float* __restrict__ out) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
         float acc = b[0];
-        for (int c = 0; c < H; ++c) acc = fmaf(X[(long long)r * H + c], w[c], acc);
+#pragma unroll 8
+        for (int c = 0; c < H; c += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(X + (long long)r * H + c);
+            acc = fmaf(x.x, w[c], acc);
+            acc = fmaf(x.y, w[c + 1], acc);
+            acc = fmaf(x.z, w[c + 2], acc);
+            acc = fmaf(x.w, w[c + 3], acc);
+        }
         out[r] = acc;
     }
 }
@@ -274,8 +443,12 @@ __global__ void g_readout(int N, const float* __restrict__ X, const float* __res
 // block sums a contiguous row range (4 row groups of H columns, combined in
 // order), then one block adds the block sums in block order
 constexpr int kMeanBlocks = 512;
-__global__ void g_col_sum_parts(int N, const float* __restrict__ X, double* __restrict__ parts) {
+__global__ void g_col_sum_parts(int n, const float* __restrict__ Xn, int m, const float* __restrict__ Xm,
+                                double* __restrict__ parts) {  // blockIdx.y: variables, constraints
     __shared__ double sh[kThreads];
+    const int N = blockIdx.y ? m : n;
+    const float* X = blockIdx.y ? Xm : Xn;
+    parts += (long long)blockIdx.y * gridDim.x * H;
     const int c = threadIdx.x % H, grp = threadIdx.x / H, ngrp = kThreads / H;
     const long long per = ((long long)N + gridDim.x - 1) / gridDim.x;
     const long long r0 = blockIdx.x * per, r1 = min((long long)N, r0 + per);
@@ -290,13 +463,28 @@ __global__ void g_col_sum_parts(int N, const float* __restrict__ X, double* __re
     }
 }
 
-__global__ void g_col_mean(int N, int nparts, const double* __restrict__ parts, float* __restrict__ out) {
-    for (int c = threadIdx.x; c < H; c += blockDim.x) {
-        double acc = 0.0;
-        for (int b = 0; b < nparts; ++b) acc += parts[(long long)b * H + c];
-        out[c] = (float)(acc / (N > 0 ? N : 1));
+// Eight columns per block (blockIdx.y: variables, constraints): the block sums
+// come to shared memory at once, then a thread per column adds them in order
+// (one load after the other it took 59 us).
+constexpr int kMeanCols = 8;
+__global__ void __launch_bounds__(kThreads) g_col_mean(int n, int m, const double* __restrict__ parts,
+                                                       float* __restrict__ out_n, float* __restrict__ out_m) {
+    __shared__ double sp[kMeanBlocks * kMeanCols];
+    const int N = blockIdx.y ? m : n, c0 = blockIdx.x * kMeanCols;
+    parts += (long long)blockIdx.y * kMeanBlocks * H + c0;
+#pragma unroll
+    for (int u = 0; u < kMeanBlocks * kMeanCols / kThreads; ++u) {
+        const int q = threadIdx.x + u * kThreads;
+        sp[q] = parts[q / kMeanCols * H + q % kMeanCols];
     }
+    __syncthreads();
+    if (threadIdx.x >= kMeanCols) return;
+    double acc = 0.0;
+#pragma unroll 16
+    for (int b = 0; b < kMeanBlocks; ++b) acc += sp[b * kMeanCols + threadIdx.x];
+    (blockIdx.y ? out_m : out_n)[c0 + threadIdx.x] = (float)(acc / (N > 0 ? N : 1));
 }
+static_assert(kMeanBlocks * kMeanCols % kThreads == 0 && H % kMeanCols == 0, "tiles of g_col_mean");
 
 // squared-error terms and d pred = 2 (pred - t) / N; partial sums per block
 __global__ void g_mse(int N, const float* __restrict__ pred, const float* __restrict__ target,
@@ -334,18 +522,76 @@ __global__ void g_outer_add(int N, const float* __restrict__ d, const float* __r
 __global__ void __launch_bounds__(kThreads) g_readout_bwd(int N, const float* __restrict__ X,
                                                           const float* __restrict__ d, float* __restrict__ part_w,
                                                           float* __restrict__ part_b) {
-    const int r0 = blockIdx.x * kRows;
-    const int rows = min(kRows, N - r0);
-    for (int c = threadIdx.x; c < H; c += blockDim.x) {
+    __shared__ __align__(16) float sX[kRows][H];
+    __shared__ float sd[kRows];
+    const long long r0 = (long long)blockIdx.x * kRows;
+    const int rows = (int)(N - r0 < kRows ? N - r0 : kRows);
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = ld4(X + (r0 + tile_row(u)) * H + tile_col(), tile_row(u) < rows);
+    if ((int)threadIdx.x < rows) sd[threadIdx.x] = d[r0 + threadIdx.x];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(&sX[tile_row(u)][tile_col()]) = v[u];
+    __syncthreads();
+    if (threadIdx.x < H) {
         float acc = 0.f;
-        for (int rr = 0; rr < rows; ++rr) acc = fmaf(d[r0 + rr], X[(long long)(r0 + rr) * H + c], acc);
-        part_w[(long long)blockIdx.x * H + c] = acc;
-    }
-    if (threadIdx.x == 0) {
+#pragma unroll 8
+        for (int rr = 0; rr < rows; ++rr) acc = fmaf(sd[rr], sX[rr][threadIdx.x], acc);
+        part_w[(long long)blockIdx.x * H + threadIdx.x] = acc;
+    } else if (threadIdx.x == H) {
         float acc = 0.f;
-        for (int rr = 0; rr < rows; ++rr) acc += d[r0 + rr];
+#pragma unroll 8
+        for (int rr = 0; rr < rows; ++rr) acc += sd[rr];
         part_b[blockIdx.x] = acc;
     }
+}
+
+// The loss and the gradient of the omega readout, in the order of the host
+// (log_omega): log omega = bw + sum mv uv + mcm uc; d uv = dlw mv, d uc = dlw mcm,
+// d bw = dlw; share[0..H) = dlw uv / n, share[H..2H) = dlw uc / m, what every
+// node's d h gets.  Kept on the device: the host took seven small copies each
+// way and three synchronisations for it (about 0.3 ms).
+__global__ void __launch_bounds__(H) g_omega_loss(int n, int m, int bx, int by, const double* __restrict__ parts,
+                                                  const float* __restrict__ mv, const float* __restrict__ mcm,
+                                                  const float* __restrict__ uv, const float* __restrict__ uc,
+                                                  const float* __restrict__ bw, double target,
+                                                  float* __restrict__ g_uv, float* __restrict__ g_uc,
+                                                  float* __restrict__ g_bw, float* __restrict__ share,
+                                                  double* __restrict__ loss) {
+    __shared__ double term[H], sums[2];
+    __shared__ float dlw_s;
+    const int c = threadIdx.x;
+    term[c] = __dadd_rn(__dmul_rn((double)mv[c], uv[c]), __dmul_rn((double)mcm[c], uc[c]));
+    if (c % 32 == 0) {  // one lane of each warp sums one side's squared errors, in block order
+        const double* p = parts + (c ? 2048 : 0);
+        const int nb = c ? by : bx;
+        double t = 0.0;
+        int b = 0;
+        for (; b + 16 <= nb; b += 16) {
+            double v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) v[u] = p[b + u];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) t += v[u];
+        }
+        for (; b < nb; ++b) t += p[b];
+        sums[c / 32] = t;
+    }
+    __syncthreads();
+    if (c == 0) {
+        double lw = bw[0];
+        for (int k = 0; k < H; ++k) lw += term[k];
+        const double ew = lw - target;
+        *loss = __dadd_rn(__dadd_rn(sums[0] / n, sums[1] / m), __dmul_rn(__dmul_rn(0.1, ew), ew));
+        dlw_s = (float)(0.2 * ew);
+        g_bw[0] = dlw_s;
+    }
+    __syncthreads();
+    const float dlw = dlw_s;
+    g_uv[c] = dlw * mv[c];
+    g_uc[c] = dlw * mcm[c];
+    share[c] = dlw * uv[c] / n;
+    share[H + c] = dlw * uc[c] / m;
 }
 
 __global__ void g_adam(long long count, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
@@ -368,11 +614,16 @@ int grid_of(long long work) {
     return b < 1 ? 1 : (int)b;
 }
 
-// blocks of the tiled dense kernels: one per 64-row tile, at most four waves' worth
-int tile_grid(long long rows) {
-    long long b = (rows + kTile - 1) / kTile;
-    if (b > 148 * 8) b = 148 * 8;
-    return b < 1 ? 1 : (int)b;
+// Y = relu(X1 W1 + X2 W2 + b): tiles of 32 rows while two blocks per SM take
+// them, then of 64; at most eight blocks per SM.
+void dense_fwd(cudaStream_t s, int N, const float* X1, int K1, const float* W1, const float* X2, const float* W2,
+               const float* b, float* Y) {
+    if (N <= 148 * 2 * 32) {
+        g_dense_fwd<32><<<std::max((N + 31) / 32, 1), kThreads, 0, s>>>(N, X1, K1, W1, X2, W2, b, Y);
+    } else {
+        const long long tiles = ((long long)N + kTile - 1) / kTile;
+        g_dense_fwd<64><<<(int)std::min<long long>(tiles, 148 * 8), kThreads, 0, s>>>(N, X1, K1, W1, X2, W2, b, Y);
+    }
 }
 
 // One instance on the device: graph, features, activations, gradients.
@@ -502,15 +753,15 @@ int reserve_ws(mc_gnn* g, int n, int m) {
     GTRY(get(&g->dhc, mH));
     GTRY(get(&g->dhv2, nH));
     GTRY(get(&g->dhc2, mH));
-    GTRY(get(&g->dag, std::max(nH, mH)));
+    GTRY(get(&g->dag, std::max({nH, mH, 2LL * H})));
     const long long blocks = (std::max(n, m) + kRows - 1) / kRows;
-    GTRY(get(&g->part, blocks * (long long)H * H + blocks * H));
+    GTRY(get(&g->part, blocks * (2LL * H * H + H)));
     void* q = nullptr;
-    GCU(cudaMalloc(&q, sizeof(double) * 4096));
+    GCU(cudaMalloc(&q, sizeof(double) * 4097));  // squared-error parts, the loss
     g->ws.push_back(q);
     g->dpart = static_cast<double*>(q);
     q = nullptr;
-    GCU(cudaMalloc(&q, sizeof(double) * kMeanBlocks * H));
+    GCU(cudaMalloc(&q, sizeof(double) * 2 * kMeanBlocks * H));
     g->ws.push_back(q);
     g->mpart = static_cast<double*>(q);
     g->cap_n = n;
@@ -775,29 +1026,23 @@ int forward(mc_gnn* g, const Instance& I) {
     const float* P = g->params;
     const Layout& L = g->L;
     const int n = I.n, m = I.m;
-    g_dense_fwd<<<tile_grid(n), kThreads, 0, s>>>(n, I.Fv, FV, P + L.Wve, nullptr, 0, nullptr,
-                                                               P + L.bve, g->hv[0], 1);
-    g_dense_fwd<<<tile_grid(m), kThreads, 0, s>>>(m, I.Fc, FC, P + L.Wce, nullptr, 0, nullptr,
-                                                               P + L.bce, g->hc[0], 1);
+    dense_fwd(s, n, I.Fv, FV, P + L.Wve, nullptr, nullptr, P + L.bve, g->hv[0]);
+    dense_fwd(s, m, I.Fc, FC, P + L.Wce, nullptr, nullptr, P + L.bce, g->hc[0]);
     for (int r = 1; r <= g->rounds; ++r) {
         // constraints gather variables: agc_i = sum_j a_ij / |A_i| hv_j
         g_aggregate<<<grid_of((long long)m * 32), kThreads, 0, s>>>(m, I.rs, I.ci, I.rv, I.rinv, nullptr,
                                                                      g->hv[r - 1], g->agc[r], 0);
-        g_dense_fwd<<<tile_grid(m), kThreads, 0, s>>>(m, g->hc[r - 1], H, P + L.Wcs[r - 1], g->agc[r], H,
-                                                                   P + L.Wcn[r - 1], P + L.bc[r - 1], g->hc[r], 1);
+        dense_fwd(s, m, g->hc[r - 1], H, P + L.Wcs[r - 1], g->agc[r], P + L.Wcn[r - 1], P + L.bc[r - 1], g->hc[r]);
         // variables gather constraints: agv_j = sum_i a_ij / |A_j| hc_i
         g_aggregate<<<grid_of((long long)n * 32), kThreads, 0, s>>>(n, I.cs, I.ri, I.cv, I.cinv, nullptr,
                                                                      g->hc[r], g->agv[r], 0);
-        g_dense_fwd<<<tile_grid(n), kThreads, 0, s>>>(n, g->hv[r - 1], H, P + L.Wvs[r - 1], g->agv[r], H,
-                                                                   P + L.Wvn[r - 1], P + L.bv[r - 1], g->hv[r], 1);
+        dense_fwd(s, n, g->hv[r - 1], H, P + L.Wvs[r - 1], g->agv[r], P + L.Wvn[r - 1], P + L.bv[r - 1], g->hv[r]);
     }
     const int R = g->rounds;
     g_readout<<<grid_of(n), kThreads, 0, s>>>(n, g->hv[R], P + L.wx, P + L.bx, g->px);
     g_readout<<<grid_of(m), kThreads, 0, s>>>(m, g->hc[R], P + L.wy, P + L.by, g->py);
-    g_col_sum_parts<<<kMeanBlocks, kThreads, 0, s>>>(n, g->hv[R], g->mpart);
-    g_col_mean<<<1, H, 0, s>>>(n, kMeanBlocks, g->mpart, g->mv);
-    g_col_sum_parts<<<kMeanBlocks, kThreads, 0, s>>>(m, g->hc[R], g->mpart);
-    g_col_mean<<<1, H, 0, s>>>(m, kMeanBlocks, g->mpart, g->mcm);
+    g_col_sum_parts<<<dim3(kMeanBlocks, 2), kThreads, 0, s>>>(n, g->hv[R], m, g->hc[R], g->mpart);
+    g_col_mean<<<dim3(H / kMeanCols, 2), kThreads, 0, s>>>(n, m, g->mpart, g->mv, g->mcm);
     GCU(cudaGetLastError());
     return MC_OK;
 }
@@ -818,14 +1063,33 @@ int log_omega(mc_gnn* g, double* out) {
     return MC_OK;
 }
 
-int weight_grad(mc_gnn* g, int N, const float* X, int K, const float* dZ, long long w_off, long long b_off) {
-    cudaStream_t s = g->stream;
+void reduce_parts(cudaStream_t s, int blocks, Parts a, Parts b, Parts c = Parts{nullptr, nullptr, 0}) {
+    const int width = a.width + b.width + c.width;
+    g_reduce_parts<<<(width + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s>>>(blocks, a, b, c);
+}
+
+// an encoder's gradients: Y = relu(X W + b), dY in model order
+int encoder_bwd(mc_gnn* g, int N, const float* X, int K, const float* Y, const float* dY, long long w_off,
+                long long b_off) {
     const int blocks = (N + kRows - 1) / kRows;
     float* pw = g->part;
     float* pb = g->part + (long long)blocks * K * H;
-    g_dense_bwd_w<<<blocks, kThreads, 0, s>>>(N, X, K, dZ, pw, b_off >= 0 ? pb : nullptr);
-    g_reduce_parts<<<grid_of(K * H), kThreads, 0, s>>>(blocks, K * H, pw, g->grads + w_off);
-    if (b_off >= 0) g_reduce_parts<<<1, H, 0, s>>>(blocks, H, pb, g->grads + b_off);
+    g_dense_bwd_w<<<blocks, kThreads, 0, g->stream>>>(N, X, K, Y, dY, pw, pb);
+    reduce_parts(g->stream, blocks, {pw, g->grads + w_off, K * H}, {pb, g->grads + b_off, H});
+    GCU(cudaGetLastError());
+    return MC_OK;
+}
+
+// an update's gradients: Y = relu(X1 W1 + X2 W2 + b) from dY, into dX1, dX2 and g->grads
+int update_bwd(mc_gnn* g, int N, const float* Y, const float* dY, const float* X1, const float* X2, long long w1,
+               long long w2, long long b, float* dX1, float* dX2) {
+    const int blocks = (N + kRows - 1) / kRows;
+    GCU(cudaFuncSetAttribute(g_update_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+    g_update_bwd<<<blocks, kThreads, kUpdateSmem, g->stream>>>(N, Y, dY, X1, X2, g->params + w1, g->params + w2, dX1,
+                                                               dX2, g->part);
+    const long long ww = (long long)blocks * H * H;
+    reduce_parts(g->stream, blocks, {g->part, g->grads + w1, H * H}, {g->part + ww, g->grads + w2, H * H},
+                 {g->part + 2 * ww, g->grads + b, H});
     GCU(cudaGetLastError());
     return MC_OK;
 }
@@ -842,77 +1106,34 @@ int loss_and_grad(mc_gnn* g, const Instance& I, double target_logw, double* loss
     const int bx = std::min(grid_of(n), 2048), by = std::min(grid_of(m), 2048);
     g_mse<<<bx, kThreads, 0, s>>>(n, g->px, g->tx, g->dx, g->dpart);
     g_mse<<<by, kThreads, 0, s>>>(m, g->py, g->ty, g->dy, g->dpart + 2048);
-    std::vector<double> parts(4096);
-    GCU(cudaMemcpyAsync(parts.data(), g->dpart, sizeof(double) * 4096, cudaMemcpyDeviceToHost, s));
-    double lw = 0.0;
-    GTRY(log_omega(g, &lw));  // synchronises
-    double lx = 0.0, ly = 0.0;
-    for (int b = 0; b < bx; ++b) lx += parts[b];
-    for (int b = 0; b < by; ++b) ly += parts[2048 + b];
-    lx /= n;
-    ly /= m;
-    const double ew = lw - target_logw;
-    *loss_out = lx + ly + 0.1 * ew * ew;
-    const float dlw = (float)(0.2 * ew);
-    // omega readout: d uv = dlw * mv, d uc = dlw * mc, d bw = dlw; d hv += dlw uv / n, d hc += dlw uc / m
-    {
-        float mv[H], mcm[H], gu[2 * H + 1];
-        GCU(cudaMemcpyAsync(mv, g->mv, sizeof mv, cudaMemcpyDeviceToHost, s));
-        GCU(cudaMemcpyAsync(mcm, g->mcm, sizeof mcm, cudaMemcpyDeviceToHost, s));
-        GCU(cudaStreamSynchronize(s));
-        for (int c = 0; c < H; ++c) {
-            gu[c] = dlw * mv[c];
-            gu[H + c] = dlw * mcm[c];
-        }
-        gu[2 * H] = dlw;
-        GCU(cudaMemcpyAsync(g->grads + L.uv, gu, sizeof(float) * H, cudaMemcpyHostToDevice, s));
-        GCU(cudaMemcpyAsync(g->grads + L.uc, gu + H, sizeof(float) * H, cudaMemcpyHostToDevice, s));
-        GCU(cudaMemcpyAsync(g->grads + L.bw, gu + 2 * H, sizeof(float), cudaMemcpyHostToDevice, s));
-        float su[2 * H];
-        GCU(cudaMemcpyAsync(su, P + L.uv, sizeof(float) * H, cudaMemcpyDeviceToHost, s));
-        GCU(cudaMemcpyAsync(su + H, P + L.uc, sizeof(float) * H, cudaMemcpyDeviceToHost, s));
-        GCU(cudaStreamSynchronize(s));
-        for (int c = 0; c < H; ++c) {
-            su[c] = dlw * su[c] / n;
-            su[H + c] = dlw * su[H + c] / m;
-        }
-        GCU(cudaMemcpyAsync(g->dag, su, sizeof(float) * 2 * H, cudaMemcpyHostToDevice, s));
-        // d hv[R] = dx wx + dlw uv / n ; d hc[R] = dy wy + dlw uc / m
-        g_outer_add<<<grid_of((long long)n * H), kThreads, 0, s>>>(n, g->dx, P + L.wx, g->dag, g->dhv, 0);
-        g_outer_add<<<grid_of((long long)m * H), kThreads, 0, s>>>(m, g->dy, P + L.wy, g->dag + H, g->dhc, 0);
-        GCU(cudaStreamSynchronize(s));  // g->dag is rewritten below
-    }
+    double* loss = g->dpart + 4096;
+    g_omega_loss<<<1, H, 0, s>>>(n, m, bx, by, g->dpart, g->mv, g->mcm, P + L.uv, P + L.uc, P + L.bw, target_logw,
+                                 g->grads + L.uv, g->grads + L.uc, g->grads + L.bw, g->dag, loss);
+    // d hv[R] = dx wx + dlw uv / n ; d hc[R] = dy wy + dlw uc / m
+    g_outer_add<<<grid_of((long long)n * H), kThreads, 0, s>>>(n, g->dx, P + L.wx, g->dag, g->dhv, 0);
+    g_outer_add<<<grid_of((long long)m * H), kThreads, 0, s>>>(m, g->dy, P + L.wy, g->dag + H, g->dhc, 0);
     // readout weights: d wx = sum dx hv, d bx = sum dx
     {
-        const int blocks = (n + kRows - 1) / kRows;
-        g_readout_bwd<<<blocks, kThreads, 0, s>>>(n, g->hv[R], g->dx, g->part, g->part + (long long)blocks * H);
-        g_reduce_parts<<<1, H, 0, s>>>(blocks, H, g->part, g->grads + L.wx);
-        g_reduce_parts<<<1, 1, 0, s>>>(blocks, 1, g->part + (long long)blocks * H, g->grads + L.bx);
-        const int bm = (m + kRows - 1) / kRows;
-        g_readout_bwd<<<bm, kThreads, 0, s>>>(m, g->hc[R], g->dy, g->part + 2LL * blocks * H + blocks,
-                                              g->part + 2LL * blocks * H + blocks + (long long)bm * H);
-        g_reduce_parts<<<1, H, 0, s>>>(bm, H, g->part + 2LL * blocks * H + blocks, g->grads + L.wy);
-        g_reduce_parts<<<1, 1, 0, s>>>(bm, 1, g->part + 2LL * blocks * H + blocks + (long long)bm * H,
-                                       g->grads + L.by);
+        const int bn = (n + kRows - 1) / kRows, bm = (m + kRows - 1) / kRows;
+        float* pn = g->part;
+        float* pm = g->part + (long long)bn * (H + 1);
+        g_readout_bwd<<<bn, kThreads, 0, s>>>(n, g->hv[R], g->dx, pn, pn + (long long)bn * H);
+        g_readout_bwd<<<bm, kThreads, 0, s>>>(m, g->hc[R], g->dy, pm, pm + (long long)bm * H);
+        reduce_parts(s, bn, {pn, g->grads + L.wx, H}, {pn + (long long)bn * H, g->grads + L.bx, 1});
+        reduce_parts(s, bm, {pm, g->grads + L.wy, H}, {pm + (long long)bm * H, g->grads + L.by, 1});
         GCU(cudaGetLastError());
     }
     // rounds, last to first.  dhv / dhc hold d h[r]; dhv2 / dhc2 build d h[r-1].
     for (int r = R; r >= 1; --r) {
         // variable update: hv[r] = relu(hv[r-1] Wvs + agv[r] Wvn + bv)
-        g_relu_bwd<<<grid_of((long long)n * H), kThreads, 0, s>>>((long long)n * H, g->hv[r], g->dhv);
-        GTRY(weight_grad(g, n, g->hv[r - 1], H, g->dhv, L.Wvs[r - 1], L.bv[r - 1]));
-        GTRY(weight_grad(g, n, g->agv[r], H, g->dhv, L.Wvn[r - 1], -1));
-        g_dense_bwd_x<<<tile_grid(n), kThreads, 0, s>>>(n, g->dhv, P + L.Wvs[r - 1], H, g->dhv2, 0);
-        g_dense_bwd_x<<<tile_grid(n), kThreads, 0, s>>>(n, g->dhv, P + L.Wvn[r - 1], H, g->dag, 0);
+        GTRY(update_bwd(g, n, g->hv[r], g->dhv, g->hv[r - 1], g->agv[r], L.Wvs[r - 1], L.Wvn[r - 1], L.bv[r - 1],
+                        g->dhv2, g->dag));
         // agv[r]_j = sum_i a_ij cinv_j hc[r]_i  ->  d hc[r]_i += sum_j a_ij cinv_j d agv_j (CSR)
         g_aggregate<<<grid_of((long long)m * 32), kThreads, 0, s>>>(m, I.rs, I.ci, I.rv, nullptr, I.cinv, g->dag,
                                                                      g->dhc, 1);
         // constraint update: hc[r] = relu(hc[r-1] Wcs + agc[r] Wcn + bc)
-        g_relu_bwd<<<grid_of((long long)m * H), kThreads, 0, s>>>((long long)m * H, g->hc[r], g->dhc);
-        GTRY(weight_grad(g, m, g->hc[r - 1], H, g->dhc, L.Wcs[r - 1], L.bc[r - 1]));
-        GTRY(weight_grad(g, m, g->agc[r], H, g->dhc, L.Wcn[r - 1], -1));
-        g_dense_bwd_x<<<tile_grid(m), kThreads, 0, s>>>(m, g->dhc, P + L.Wcs[r - 1], H, g->dhc2, 0);
-        g_dense_bwd_x<<<tile_grid(m), kThreads, 0, s>>>(m, g->dhc, P + L.Wcn[r - 1], H, g->dag, 0);
+        GTRY(update_bwd(g, m, g->hc[r], g->dhc, g->hc[r - 1], g->agc[r], L.Wcs[r - 1], L.Wcn[r - 1], L.bc[r - 1],
+                        g->dhc2, g->dag));
         // agc[r]_i = sum_j a_ij rinv_i hv[r-1]_j  ->  d hv[r-1]_j += sum_i a_ij rinv_i d agc_i (CSC)
         g_aggregate<<<grid_of((long long)n * 32), kThreads, 0, s>>>(n, I.cs, I.ri, I.cv, nullptr, I.rinv, g->dag,
                                                                      g->dhv2, 1);
@@ -920,11 +1141,10 @@ int loss_and_grad(mc_gnn* g, const Instance& I, double target_logw, double* loss
         std::swap(g->dhc, g->dhc2);
     }
     // encoders
-    g_relu_bwd<<<grid_of((long long)n * H), kThreads, 0, s>>>((long long)n * H, g->hv[0], g->dhv);
-    GTRY(weight_grad(g, n, I.Fv, FV, g->dhv, L.Wve, L.bve));
-    g_relu_bwd<<<grid_of((long long)m * H), kThreads, 0, s>>>((long long)m * H, g->hc[0], g->dhc);
-    GTRY(weight_grad(g, m, I.Fc, FC, g->dhc, L.Wce, L.bce));
-    GCU(cudaGetLastError());
+    GTRY(encoder_bwd(g, n, I.Fv, FV, g->hv[0], g->dhv, L.Wve, L.bve));
+    GTRY(encoder_bwd(g, m, I.Fc, FC, g->hc[0], g->dhc, L.Wce, L.bce));
+    GCU(cudaMemcpyAsync(loss_out, loss, sizeof(double), cudaMemcpyDeviceToHost, s));
+    GCU(cudaStreamSynchronize(s));
     return MC_OK;
 }
 
