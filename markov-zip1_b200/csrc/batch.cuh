@@ -439,6 +439,7 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     CU(cudaMemsetAsync(counters, 0, sizeof(int) * 4, s));
     // one kind of array after the other, so that the LPs' pieces follow one another
     Staging& up = ctx.staging;
+    up.begin();
     int* ends = static_cast<int*>(at(o_ends));
     for (int b = 0; b < count; ++b) {
         if (!lps[b].col_start) return cuda_fail(cudaErrorInvalidValue, "column pointers", __LINE__);

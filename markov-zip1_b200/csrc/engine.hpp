@@ -85,6 +85,8 @@ struct Staging {
     char* run_dst = nullptr;
 
     void free();
+    // start of a call: what an earlier call left unsent when it failed is dropped
+    void begin() { run_bytes = 0; }
     int ready();
     int turn(cudaStream_t s);  // to the other buffer
     int flush(cudaStream_t s);

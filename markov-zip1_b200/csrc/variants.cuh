@@ -1595,6 +1595,7 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     double* wy = any_wy ? static_cast<double*>(at(o_wy)) : nullptr;
     std::vector<int> hw(2 * (size_t)count, 0);
     Staging& up = ctx.staging;
+    up.begin();
     for (int b = 0; b < count; ++b)
         TRY(up.put(s, lo_in + (size_t)b * n, (var_lower && var_lower[b]) ? var_lower[b] : base->var_lower, sizeof(double) * n));
     for (int b = 0; b < count; ++b)

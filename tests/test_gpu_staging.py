@@ -71,3 +71,24 @@ def test_invalid_member_is_found_in_its_own_numbering(gpu_ctx):
             bad.row_index[[0, 1]] = bad.row_index[[1, 0]]
         with pytest.raises(ValueError, match="invalid CSC matrix in the batch"):
             gpu_ctx.solve_batch(models, PdlpOptions())
+
+
+def test_call_after_one_that_failed_between_its_uploads(gpu_ctx):
+    class NoColumns(mcpdlp.Model):
+        def to_struct(self):
+            s = super().to_struct()
+            s.col_start = None
+            return s
+
+    good = [generators.random_lp(60 + i, 70 + 9 * i, 200, 4) for i in range(3)]
+    m = good[1]
+    broken = NoColumns(m.num_rows, m.num_cols, m.col_start, m.row_index, m.value, m.objective, m.var_lower,
+                       m.var_upper, m.row_lower, m.row_upper)
+    o = PdlpOptions(max_iterations=120)
+    o.set_tolerance(1e-13)
+    expect = gpu_ctx.solve_batch(good, o)
+    with pytest.raises(Exception):
+        gpu_ctx.solve_batch([good[0], broken, good[2]], o)
+    for r, e in zip(gpu_ctx.solve_batch(good, o), expect):
+        np.testing.assert_array_equal(r.primal, e.primal)
+        np.testing.assert_array_equal(r.dual, e.dual)
