@@ -1217,6 +1217,7 @@ int finish_session(Ctx& ctx, double* x_out, double* y_out, mc_pdlp_result* res) 
     CU(cudaStreamSynchronize(s));
     TRY(ctx.drain_profile());
     const DevState& DS = ctx.h_state[3];
+    if (DS.fault) return set_error(MC_ERR_CUDA, "a wait of a cooperative kernel timed out");
     if (trace && trace_cap > 0) {
         const long long cnt = std::min<long long>(DS.checks, trace_cap);
         trace->count = cnt;
