@@ -225,19 +225,19 @@ __device__ __forceinline__ double slice_dot_plain(const int* idx, const double* 
 // corrections (P. Markstein, IBM J. Res. Dev. 34, 1990).  a y is within 1.5
 // units of the last place of a / b; the first correction brings it within
 // one, the second rounds it correctly, as every remainder a - q b is then
-// exact.  Holds while no intermediate under- or overflows; outside a safe
-// range of |a| it divides.  b is an iteration count or a step size, so its
-// own range is never an issue for the values below.
+// exact.  Holds while no intermediate under- or overflows: outside a safe
+// range of |a| and y it divides.  (b is an iteration count or a step size; a
+// step size of an unscaled model can be anything, 0 and infinity included.)
 __device__ __forceinline__ double div_recip(double a, double b, double y) {
     const double m = fabs(a);
-    if (!(m < 1e150) || (m < 1e-150 && m != 0.0)) return __ddiv_rn(a, b);
+    if (!(y > 1e-100 && y < 1e150) || !(m < 1e150) || (m < 1e-150 && m != 0.0)) return __ddiv_rn(a, b);
     double q = __dmul_rn(a, y);
     q = fma(fma(-q, b, a), y, q);
     return fma(fma(-q, b, a), y, q);
 }
 __device__ __forceinline__ float div_recip(float a, float b, float y) {
     const float m = fabsf(a);
-    if (!(m < 1e15f) || (m < 1e-15f && m != 0.f)) return __fdiv_rn(a, b);
+    if (!(y > 1e-15f && y < 1e15f) || !(m < 1e15f) || (m < 1e-15f && m != 0.f)) return __fdiv_rn(a, b);
     float q = __fmul_rn(a, y);
     q = fmaf(fmaf(-q, b, a), y, q);
     return fmaf(fmaf(-q, b, a), y, q);

@@ -149,3 +149,27 @@ def test_step_size_and_restart_options(gpu_ctx, oracle):
             assert res.iterations == cpu.iterations
             assert rel(res.primal, cpu.primal) <= 1e-9, kw
             assert rel(res.dual, cpu.dual) <= 1e-9, kw
+
+
+@pytest.mark.parametrize("m,n", [(40, 90), (1500, 9000)])  # cluster and grid form
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+def test_unscaled_rows_of_any_magnitude(gpu_ctx, m, n, precision):
+    """Without equilibration a row's step size may be any number: the division
+    by it must be the streaming kernels' one where its reciprocal leaves the
+    safe range."""
+    model = generators.random_lp(31, m, n, 5)
+    top = 20 if precision == "fp32_refine" else 60
+    scale = 10.0 ** np.linspace(-top, top, m)[np.random.default_rng(3).permutation(m)]
+    model.value = model.value * scale[model.row_index]
+    model.row_lower, model.row_upper = model.row_lower * scale, model.row_upper * scale + scale
+    # no step-size rule and no restart check: nothing depends on a reduction's order
+    o = PdlpOptions(max_iterations=37, precision=Precision[precision], ruiz_scaling=False, adaptive_step_size=False,
+                    initial_primal_weight=1.0)
+    o.set_tolerance(1e-14)
+    res = gpu_ctx.solve(model, o)
+    o.lanes_per_column, o.lanes_per_row = lanes(model.nnz / n), lanes(model.nnz / m)
+    ref = gpu_ctx.solve_batch([model], o)[0]
+    for a, b in ((res.primal, ref.primal), (res.dual, ref.dual)):
+        ok = np.isfinite(b)
+        np.testing.assert_array_equal(np.isfinite(a), ok)
+        np.testing.assert_allclose(np.asarray(a)[ok], np.asarray(b)[ok], rtol=1e-11, atol=0)
