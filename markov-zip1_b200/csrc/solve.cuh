@@ -114,12 +114,11 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
     inclusive_scan(ctx, csr_start, m + 1, scan_tmp);  // the m+1 counts
     if (nnz == 0) return ctx.launch_check("build_csr");
     const int nb_n = (int)((n + kBlock - 1) / kBlock);
-    const int nb_m = (int)((m + kBlock - 1) / kBlock);
     ctx.begin_launch(MC_KERNEL_SETUP);
     k_scatter_rows<<<nb_n, kBlock, 0, s>>>(n, csc_start, csc_row, csc_val, csr_start, cursor, csr_col, csr_val);
     ctx.end_launch();
     ctx.begin_launch(MC_KERNEL_SETUP);
-    k_sort_short_rows<<<nb_m, kBlock, 0, s>>>(m, csr_start, csr_col, csr_val, long_rows, counters);
+    k_sort_short_rows<<<(int)(((long long)m * 32 + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, csr_start, csr_col, csr_val, long_rows, counters);
     ctx.end_launch();
     ctx.begin_launch(MC_KERNEL_SETUP);
     k_max_line<<<blocks_for(ctx, m, kBlock), kBlock, 0, s>>>(m, csr_start, counters + 1);
