@@ -317,6 +317,10 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     for (int b = 0; b < count; ++b) {
         std::memset(&results[b], 0, sizeof(mc_pdlp_result));
         TRY(validate_lp(&lps[b]));
+        // an LP without columns has no thread in kb_validate_csc, one without rows no row to hold an entry
+        if (lps[b].nnz > 0 && (lps[b].num_cols == 0 || lps[b].num_rows == 0))
+            return set_error(MC_ERR_INVALID_ARGUMENT, "invalid CSC matrix in the batch (LP %d has entries but no %s)", b,
+                             lps[b].num_cols == 0 ? "columns" : "rows");
         col_off[b + 1] = col_off[b] + lps[b].num_cols;
         row_off[b + 1] = row_off[b] + lps[b].num_rows;
         nnz_off[b + 1] = nnz_off[b] + lps[b].nnz;
@@ -444,7 +448,7 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
     for (int b = 0; b < count; ++b) {
         if (!lps[b].col_start) return cuda_fail(cudaErrorInvalidValue, "column pointers", __LINE__);
         TRY(up.put(s, cs + col_off[b], lps[b].col_start, sizeof(int) * (size_t)lps[b].num_cols));
-        if (lps[b].num_cols > 0 && lps[b].nnz > 0)
+        if (lps[b].num_cols > 0)
             TRY(up.put(s, ends + b, lps[b].col_start + lps[b].num_cols, sizeof(int)));
     }
     for (int b = 0; b < count; ++b) TRY(up.put(s, ri + nnz_off[b], lps[b].row_index, sizeof(int) * (size_t)lps[b].nnz));

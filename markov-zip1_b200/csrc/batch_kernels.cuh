@@ -615,6 +615,8 @@ __device__ __forceinline__ int packed_lp(const int* __restrict__ off, int nlp, l
 
 // k_validate_csc for every LP of the batch, in the LPs' own numbering (before
 // kb_shift_indices); ends[lp] is the last entry of the LP's column pointers.
+// An LP without entries is looked at like any other: its column pointers are
+// shifted and followed too.
 __global__ void kb_validate_csc(int n, int nlp, const int* __restrict__ col_off, const int* __restrict__ row_off,
                                 const int* __restrict__ nnz_off, const int* __restrict__ ends,
                                 const int* __restrict__ col_start, const int* __restrict__ row_index,
@@ -623,7 +625,6 @@ __global__ void kb_validate_csc(int n, int nlp, const int* __restrict__ col_off,
     if (j >= n) return;
     const int lp = packed_lp(col_off, nlp, j);
     const int nnz = nnz_off[lp + 1] - nnz_off[lp], m = row_off[lp + 1] - row_off[lp];
-    if (nnz == 0) return;
     const bool last = j + 1 == col_off[lp + 1];
     const int b = col_start[j], e = last ? ends[lp] : col_start[j + 1];
     if (j == col_off[lp] && b != 0) atomicOr(bad, 1);
