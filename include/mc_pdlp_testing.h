@@ -11,9 +11,9 @@
 extern "C" {
 #endif
 
-/* The next `count` device-arena allocations of any context fail as if
- * cudaMalloc had returned cudaErrorMemoryAllocation: the solve returns
- * MC_ERR_OUT_OF_MEMORY and no device memory is touched.  0 disarms. */
+/* The next `count` allocations of a context's device arena or of a network's
+ * workspace fail as if cudaMalloc had returned cudaErrorMemoryAllocation: the
+ * call returns MC_ERR_OUT_OF_MEMORY and no device memory is touched.  0 disarms. */
 int mc_test_inject_alloc_failures(int count);
 
 #ifdef __cplusplus

@@ -70,6 +70,13 @@ int check_device(int device) {
 }
 
 // ----------------------------------------------------------------- arena
+// Whether this allocation is one that a test asked to fail.
+bool injected_alloc_failure() {
+    if (g_inject_alloc_failures <= 0) return false;
+    --g_inject_alloc_failures;
+    return true;
+}
+
 int Arena::reserve(size_t bytes) {
     if (bytes <= capacity) return MC_OK;
     if (base) {
@@ -77,10 +84,8 @@ int Arena::reserve(size_t bytes) {
         base = nullptr;
         capacity = 0;
     }
-    if (g_inject_alloc_failures > 0) {
-        --g_inject_alloc_failures;
+    if (injected_alloc_failure())
         return set_error(MC_ERR_OUT_OF_MEMORY, "injected allocation failure (%zu bytes)", bytes);
-    }
     cudaError_t e = cudaMalloc(&base, bytes);
     if (e != cudaSuccess) {
         base = nullptr;

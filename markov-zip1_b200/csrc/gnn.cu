@@ -40,6 +40,7 @@ Ctx* aux_ctx_create(int device);
 void aux_ctx_destroy(Ctx* c);
 int aux_csr(Ctx* c, int m, int n, long long nnz, const int* cs, const int* ri, const double* v, int* rs, int* ci,
             double* rv);
+bool injected_alloc_failure();
 }
 
 namespace {
@@ -701,7 +702,7 @@ struct mc_gnn {
     float *part = nullptr;
     double* dpart = nullptr;
     double* mpart = nullptr;  // block sums of the readout's column means
-    long long cap_n = -1, cap_m = -1;
+    long long cap_n = -1, cap_m = -1;  // what the workspace is sized for; -1: there is none
     std::vector<void*> ws;
     mc::Ctx* aux = nullptr;  // the engine's transpose, for large instances
     ~mc_gnn() {
@@ -718,21 +719,32 @@ struct mc_gnn {
 
 namespace {
 
+// One buffer of the workspace; its list frees it.
+template <class T>
+int ws_alloc(std::vector<void*>& list, T** p, long long count) {
+    void* q = nullptr;
+    const size_t bytes = sizeof(T) * (size_t)std::max<long long>(count, 1);
+    if (mc::injected_alloc_failure())
+        return mc::set_error(MC_ERR_OUT_OF_MEMORY, "injected allocation failure (%zu bytes)", bytes);
+    GCU(cudaMalloc(&q, bytes));
+    list.push_back(q);
+    *p = static_cast<T*>(q);
+    return MC_OK;
+}
+
 int reserve_ws(mc_gnn* g, int n, int m) {
     if (n <= g->cap_n && m <= g->cap_m) return MC_OK;
+    // Without the old buffers there is no workspace until every new one is
+    // there: a failure below must not leave the old size standing for freed
+    // pointers.
+    g->cap_n = g->cap_m = -1;
     for (void* p : g->ws) cudaFree(p);
     g->ws.clear();
     g->hv.assign(g->rounds + 1, nullptr);
     g->hc.assign(g->rounds + 1, nullptr);
     g->agv.assign(g->rounds + 1, nullptr);
     g->agc.assign(g->rounds + 1, nullptr);
-    auto get = [&](float** p, long long count) -> int {
-        void* q = nullptr;
-        GCU(cudaMalloc(&q, sizeof(float) * (size_t)std::max<long long>(count, 1)));
-        g->ws.push_back(q);
-        *p = static_cast<float*>(q);
-        return MC_OK;
-    };
+    auto get = [&](auto** p, long long count) { return ws_alloc(g->ws, p, count); };
     const long long nH = (long long)n * H, mH = (long long)m * H;
     for (int r = 0; r <= g->rounds; ++r) {
         GTRY(get(&g->hv[r], nH));
@@ -756,14 +768,8 @@ int reserve_ws(mc_gnn* g, int n, int m) {
     GTRY(get(&g->dag, std::max({nH, mH, 2LL * H})));
     const long long blocks = (std::max(n, m) + kRows - 1) / kRows;
     GTRY(get(&g->part, blocks * (2LL * H * H + H)));
-    void* q = nullptr;
-    GCU(cudaMalloc(&q, sizeof(double) * 4097));  // squared-error parts, the loss
-    g->ws.push_back(q);
-    g->dpart = static_cast<double*>(q);
-    q = nullptr;
-    GCU(cudaMalloc(&q, sizeof(double) * 2 * kMeanBlocks * H));
-    g->ws.push_back(q);
-    g->mpart = static_cast<double*>(q);
+    GTRY(get(&g->dpart, 4097));  // squared-error parts, the loss
+    GTRY(get(&g->mpart, 2 * kMeanBlocks * H));
     g->cap_n = n;
     g->cap_m = m;
     return MC_OK;
