@@ -702,13 +702,15 @@ struct mc_gnn {
     float *part = nullptr;
     double* dpart = nullptr;
     double* mpart = nullptr;  // block sums of the readout's column means
-    long long cap_n = -1, cap_m = -1;  // what the workspace is sized for; -1: there is none
-    std::vector<void*> ws;
+    // what the workspaces of the forward pass and of the gradient are sized for; -1: there is none
+    long long cap_n = -1, cap_m = -1, grad_cap_n = -1, grad_cap_m = -1;
+    std::vector<void*> ws, grad_ws;
     mc::Ctx* aux = nullptr;  // the engine's transpose, for large instances
     ~mc_gnn() {
         if (device >= 0) cudaSetDevice(device);
         if (aux) mc::aux_ctx_destroy(aux);
-        for (void* p : ws) cudaFree(p);
+        for (auto* list : {&ws, &grad_ws})
+            for (void* p : *list) cudaFree(p);
         cudaFree(params);
         cudaFree(grads);
         cudaFree(m1);
@@ -754,13 +756,27 @@ int reserve_ws(mc_gnn* g, int n, int m) {
     }
     GTRY(get(&g->px, n));
     GTRY(get(&g->py, m));
+    GTRY(get(&g->mv, H));
+    GTRY(get(&g->mcm, H));
+    GTRY(get(&g->logw, 4));
+    GTRY(get(&g->mpart, 2 * kMeanBlocks * H));
+    g->cap_n = n;
+    g->cap_m = m;
+    return MC_OK;
+}
+
+// What only a gradient needs (at 5M columns and 2M rows 7.5 GB; a prediction does without).
+int reserve_grad_ws(mc_gnn* g, int n, int m) {
+    if (n <= g->grad_cap_n && m <= g->grad_cap_m) return MC_OK;
+    g->grad_cap_n = g->grad_cap_m = -1;
+    for (void* p : g->grad_ws) cudaFree(p);
+    g->grad_ws.clear();
+    auto get = [&](auto** p, long long count) { return ws_alloc(g->grad_ws, p, count); };
+    const long long nH = (long long)n * H, mH = (long long)m * H;
     GTRY(get(&g->dx, n));
     GTRY(get(&g->dy, m));
     GTRY(get(&g->tx, n));
     GTRY(get(&g->ty, m));
-    GTRY(get(&g->mv, H));
-    GTRY(get(&g->mcm, H));
-    GTRY(get(&g->logw, 4));
     GTRY(get(&g->dhv, nH));
     GTRY(get(&g->dhc, mH));
     GTRY(get(&g->dhv2, nH));
@@ -769,9 +785,8 @@ int reserve_ws(mc_gnn* g, int n, int m) {
     const long long blocks = (std::max(n, m) + kRows - 1) / kRows;
     GTRY(get(&g->part, blocks * (2LL * H * H + H)));
     GTRY(get(&g->dpart, 4097));  // squared-error parts, the loss
-    GTRY(get(&g->mpart, 2 * kMeanBlocks * H));
-    g->cap_n = n;
-    g->cap_m = m;
+    g->grad_cap_n = n;
+    g->grad_cap_m = m;
     return MC_OK;
 }
 
@@ -1288,6 +1303,7 @@ int mc_gnn_loss_and_grad(mc_gnn* g, const mc_lp* lp, const double* x_target, con
     Instance I(g->device, g->stream);
     GTRY(load_instance(g, lp, I));
     GTRY(reserve_ws(g, I.n, I.m));
+    GTRY(reserve_grad_ws(g, I.n, I.m));
     GTRY(set_targets(g, I, x_target, y_target));
     GTRY(loss_and_grad(g, I, log_omega_target, loss));
     // the network works on its own non-blocking stream: read after it drains
