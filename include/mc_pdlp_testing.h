@@ -7,6 +7,8 @@
 #ifndef MC_PDLP_TESTING_H
 #define MC_PDLP_TESTING_H
 
+#include "mc_pdlp.h"
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -15,6 +17,12 @@ extern "C" {
  * workspace fail as if cudaMalloc had returned cudaErrorMemoryAllocation: the
  * call returns MC_ERR_OUT_OF_MEMORY and no device memory is touched.  0 disarms. */
 int mc_test_inject_alloc_failures(int count);
+
+/* How many polls the waits inside the context's cooperative kernels take before
+ * a kernel gives up and its call returns MC_ERR_CUDA: at a barrier of the grid,
+ * and for one entry that another block writes.  0 restores a default (seconds).
+ * A few polls make an ordinary wait run out. */
+int mc_test_set_wait_limits(mc_pdlp_ctx* ctx, unsigned barrier_polls, unsigned entry_polls);
 
 #ifdef __cplusplus
 }

@@ -181,7 +181,13 @@ __device__ __forceinline__ double reduce_partials(const double* p, int count, do
     return block_reduce(v, scratch, op);
 }
 
-constexpr unsigned kSpinLimit = 1u << 23;  // polls of one wait (seconds) before a thread gives up
+constexpr unsigned kSpinLimit = 1u << 23;  // polls of one wait (seconds) before a thread gives up; the default
+
+// How many polls the waits of a cooperative kernel may take.
+struct WaitLimits {
+    unsigned barrier = kSpinLimit;  // at a barrier of the whole grid
+    unsigned entry = kSpinLimit;    // for one gathered entry or partial of another block
+};
 
 // Barrier across the blocks of a launch, in two halves: the hardware barrier of
 // a cluster (CL), or for a cooperative launch a counter, zeroed before it, that
@@ -190,7 +196,8 @@ template <bool CL>
 struct BlockBarrier {
     unsigned* counter;
     unsigned target;
-    bool alone;  // a cluster of one block
+    unsigned limit;  // polls of one wait
+    bool alone;      // a cluster of one block
     __device__ __forceinline__ void arrive() {
         if (CL) {
             if (!alone) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -213,7 +220,7 @@ struct BlockBarrier {
             do {
                 asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
                 if (v - target < (1u << 30)) break;
-                ok = ++spins < kSpinLimit;
+                ok = ++spins < limit;
             } while (ok);
             __threadfence();
         }

@@ -106,6 +106,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     Arena arena;
     Staging staging;
+    WaitLimits limits;
     DevState* h_state = nullptr;  // pinned, [4]
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr;
     cudaEvent_t ev_poll[2] = {nullptr, nullptr};

@@ -109,6 +109,7 @@ template <class T, int STRIDE>
 struct FromTagged {
     const Tagged<T>* v;
     Tag want;
+    unsigned limit;
     bool& bad;
     __device__ static T scalar();
     template <int N>
@@ -125,7 +126,7 @@ struct FromTagged {
 #pragma unroll
             for (int q = 0; q < N; ++q)
                 if (tag[q] != want) ld_tagged(v + (long long)STRIDE * i[q], a[q], tag[q]);
-            bad = ++spins > kSpinLimit;
+            bad = ++spins > limit;
         }
     }
 };
@@ -254,6 +255,7 @@ struct PersistArgs {
     int g_col, g_row, g_probe;  // lanes per line
     int smem_bytes;     // dynamic shared memory of the launch
     unsigned* counter;  // arrivals at the grid barrier, zeroed before the launch
+    WaitLimits limits;
     // grid form: tagged (x-bar, dx) pairs [2n] and y [2m, every other one used]:
     // one 32-byte sector per column and row, whose owner is its only writer
     void *tx, *ty;
@@ -360,11 +362,11 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
     // dots of the group's lines against the gathered vectors
     auto from = [&](T* shared, Tagged<T>* tagged, Tag want) {
         if constexpr (CL) return FromShared<T>{shared};
-        else return FromTagged<T, 2>{tagged, want, bad};
+        else return FromTagged<T, 2>{tagged, want, A.limits.entry, bad};
     };
     auto pairs = [&]() {
         if constexpr (CL) return PairsFromShared<T>{xbuf, dbuf};
-        else return PairsFromTagged<T>{{tx, now, bad}};
+        else return PairsFromTagged<T>{{tx, now, A.limits.entry, bad}};
     };
     // The whole of a short vector into shared memory.  Entries that no line of
     // this block needs may already be ahead of `want`: any tag from it on ends
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             ld_tagged(tagged + 2LL * q, v, tag);
             while (tag < want && !bad) {
                 ld_tagged(tagged + 2LL * q, v, tag);
-                bad = ++spins > kSpinLimit;
+                bad = ++spins > A.limits.entry;
             }
             to[q] = v;
         }
@@ -432,7 +434,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
         if (tid < 16)
             st_tagged(A.tp + (16 + (tid & 8)) * kPersistMaxBlocks + b * 8 + (tid & 7), 0.0, Tag(0));
     }
-    BlockBarrier<CL> bar{A.counter, 0u, nb == 1};
+    BlockBarrier<CL> bar{A.counter, 0u, A.limits.barrier, nb == 1};
     // an entry of a gathered vector to every block's copy, the group's lanes
     // sharing the blocks
     auto spread = [&](T* buf, int at_, T v, int sub, int G) {
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
                     int r_[N];
 #pragma unroll
                     for (int r = 0; r < N; ++r) r_[r] = min(r * 32 + lane, nb - 1);
-                    FromTagged<double, 1>{set + q * kPersistMaxBlocks, rnum, bad}.get(r_, o);
+                    FromTagged<double, 1>{set + q * kPersistMaxBlocks, rnum, A.limits.entry, bad}.get(r_, o);
 #pragma unroll
                     for (int r = 0; r < N; ++r)
                         if (r * 32 + lane < nb) t = q < NMAX ? maxv(t, o[r]) : t + o[r];
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
                 } else if (lane == 0) {
                     const int at_[1] = {q};
                     double o[1];
-                    FromTagged<double, 1>{result + b * 8, rnum, bad}.get(at_, o);
+                    FromTagged<double, 1>{result + b * 8, rnum, A.limits.entry, bad}.get(at_, o);
                     t = o[0];
                 }
                 if (lane == 0) sums[q] = t;
@@ -646,7 +648,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
         auto averages = [&](T* shared, const double* base, const T* corr, const Tagged<double>* tagged) {
             if constexpr (SH) return FromShared<T>{shared};
             else if constexpr (CL) return FromBase<T>{base, corr};
-            else return FromTagged<double, 1>{tagged, now, bad};
+            else return FromTagged<double, 1>{tagged, now, A.limits.entry, bad};
         };
         RowTerms rt;
         ColTerms ct;

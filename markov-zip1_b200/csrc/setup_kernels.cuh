@@ -341,9 +341,10 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
 }
 
 __global__ void __launch_bounds__(kBlock) k_ruiz(RuizSide C, RuizSide R, long long passes, double tolerance, int nlp,
-                                                 unsigned long long* errs, unsigned* counter, DevState* st) {
+                                                 unsigned long long* errs, unsigned* counter, unsigned limit,
+                                                 DevState* st) {
     __shared__ double scratch[32];
-    BlockBarrier<false> bar{counter, 0u, false};
+    BlockBarrier<false> bar{counter, 0u, limit, false};
     ruiz_side<true>(C, nullptr, 0, errs, 0, 0, 1, nlp, tolerance, scratch);
     ruiz_side<true>(R, nullptr, 0, errs, 0, 0, 0, nlp, tolerance, scratch);
     int set = 0;

@@ -165,7 +165,7 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long passes
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     ctx.begin_launch(MC_KERNEL_SETUP);
-    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, st));
+    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, ctx.limits.barrier, st));
     ctx.end_launch();
     return ctx.launch_check("ruiz");
 }
@@ -337,6 +337,7 @@ int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int rem, int
     A.g_probe = eng.pl.g_probe;
     A.smem_bytes = pk.smem;
     A.counter = pk.counter;
+    A.limits = ctx.limits;
     A.tx = pk.tx;
     A.ty = pk.ty;
     A.stage_y = pk.stage_y;
@@ -614,7 +615,7 @@ int loop_chunks(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long ma
         if (L.inflight >= poll_every || L.chunk + 1 == stop) {
             if (L.have_prev) {
                 CU(cudaEventSynchronize(ctx.ev_poll[L.ev_idx ^ 1]));
-                if (ctx.h_state[L.ev_idx ^ 1].done) L.done = true;
+                if (ctx.h_state[L.ev_idx ^ 1].done || ctx.h_state[L.ev_idx ^ 1].fault) L.done = true;
                 L.cls = eng.shape_class(ctx.h_state[L.ev_idx ^ 1]);
             }
             CU(cudaMemcpyAsync(&ctx.h_state[L.ev_idx], st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
