@@ -24,6 +24,11 @@ int mc_test_inject_alloc_failures(int count);
  * A few polls make an ordinary wait run out. */
 int mc_test_set_wait_limits(mc_pdlp_ctx* ctx, unsigned barrier_polls, unsigned entry_polls);
 
+/* In the persistent loop's form of one block per SM this block behaves as if a
+ * wait of its had run out before its first gather: it waits for nothing and
+ * goes on with whatever it reads, until the next reduction.  -1: none. */
+int mc_test_fail_block(mc_pdlp_ctx* ctx, int block);
+
 #ifdef __cplusplus
 }
 #endif

@@ -536,4 +536,11 @@ int mc_test_set_wait_limits(mc_pdlp_ctx* c, unsigned barrier_polls, unsigned ent
     return MC_OK;
 }
 
+int mc_test_fail_block(mc_pdlp_ctx* c, int block) {
+    Ctx* ctx = reinterpret_cast<Ctx*>(c);
+    if (!ctx) return set_error(MC_ERR_INVALID_ARGUMENT, "context is NULL");
+    ctx->fail_block = block;
+    return MC_OK;
+}
+
 }  // extern "C"

@@ -107,6 +107,7 @@ struct Ctx {
     Arena arena;
     Staging staging;
     WaitLimits limits;
+    int fail_block = -1;  // persistent loop: a block whose waits run out at once (tests)
     DevState* h_state = nullptr;  // pinned, [4]
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr;
     cudaEvent_t ev_poll[2] = {nullptr, nullptr};

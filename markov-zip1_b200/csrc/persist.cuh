@@ -40,6 +40,7 @@
 #include "mixed.cuh"
 
 #include <cooperative_groups.h>
+#include <cstddef>
 
 namespace mc {
 
@@ -53,6 +54,7 @@ constexpr int kPersistPartials = 2 * 2 * 8 * kPersistMaxBlocks;  // tagged parti
 // nonzeros).  Every bit of the word is used: a load of which only parts are
 // used may be narrowed and is then no longer one access.
 using Tag = unsigned long long;
+constexpr Tag kFailed = 1ull << 63;  // in the tag of a reduction's partial or sum: a wait has run out
 template <class T>
 struct alignas(16) Tagged {
     unsigned long long value;
@@ -105,7 +107,7 @@ struct FromBase {  // mixed form, CL: base plus averaged correction from global 
         for (int q = 0; q < N; ++q) a[q] = __ldcg(base + i[q]) + (double)__ldcg(corr + i[q]);
     }
 };
-template <class T, int STRIDE>
+template <class T, int STRIDE, bool REDUCTION = false>
 struct FromTagged {
     const Tagged<T>* v;
     Tag want;
@@ -121,12 +123,20 @@ struct FromTagged {
         while (true) {
             bool all = true;
 #pragma unroll
-            for (int q = 0; q < N; ++q) all = all && tag[q] == want;
+            for (int q = 0; q < N; ++q) all = all && (REDUCTION ? tag[q] & ~kFailed : tag[q]) == want;
+            if (REDUCTION && all) {
+#pragma unroll
+                for (int q = 0; q < N; ++q) bad = bad || (tag[q] & kFailed);
+            }
             if (all || bad) return;
 #pragma unroll
             for (int q = 0; q < N; ++q)
                 if (tag[q] != want) ld_tagged(v + (long long)STRIDE * i[q], a[q], tag[q]);
             bad = ++spins > limit;
+            if (!REDUCTION) {  // overwritten already: its owner did not wait for this block
+#pragma unroll
+                for (int q = 0; q < N; ++q) bad = bad || tag[q] > want;
+            }
         }
     }
 };
@@ -256,6 +266,7 @@ struct PersistArgs {
     int smem_bytes;     // dynamic shared memory of the launch
     unsigned* counter;  // arrivals at the grid barrier, zeroed before the launch
     WaitLimits limits;
+    int fail_block;     // -1, or a block whose waits run out at once (tests)
     // grid form: tagged (x-bar, dx) pairs [2n] and y [2m, every other one used]:
     // one 32-byte sector per column and row, whose owner is its only writer
     void *tx, *ty;
@@ -303,7 +314,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
     namespace cg = cooperative_groups;
     if (tid == 0) S = *P.st;
     __syncthreads();
-    if (S.done) return;  // every block reads the same state
+    if (S.done || S.fault) return;  // every block reads the same state
     const int Gc = A.g_col, Gr = A.g_row, Gp = A.g_probe;
     const int sub_c = tid & (Gc - 1), sub_r = tid & (Gr - 1);
     // the block's lines: equal runs, at most blockDim / G of them (the launch's rule)
@@ -358,7 +369,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
     Tagged<T>* ty = static_cast<Tagged<T>*>(A.ty);
     Tag now = 0;  // number of the iteration within the launch (a check counts as one)
     Tag rnum = 0;  // number of the reduction
-    bool bad = false;
+    bool bad = !CL && b == A.fail_block;
     // dots of the group's lines against the gathered vectors
     auto from = [&](T* shared, Tagged<T>* tagged, Tag want) {
         if constexpr (CL) return FromShared<T>{shared};
@@ -452,8 +463,8 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             const double t = warp_fold(v[q], q < NMAX);
             if (lane == 0) red[q][warp] = t;
         }
-        __syncthreads();
         if constexpr (CL) {
+            __syncthreads();
             for (int q = warp; q < COUNT; q += W) {
                 const double t = warp_fold(lane < W ? red[q][lane] : 0.0, q < NMAX);
                 if (nb == 1) {
@@ -473,10 +484,15 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             // reuses a set only after every block has read it (they all have
             // contributed to the reduction in between)
             ++rnum;
+            // A block in which a wait has run out says so with its partials, and
+            // block 0 with the sums: no block goes on with what it computed
+            // from entries that had not come.
+            bad = __syncthreads_or(bad);
+            const Tag mark = bad ? rnum | kFailed : rnum;
             Tagged<double>* set = A.tp + (size_t)(rnum & 1) * 8 * kPersistMaxBlocks;
             for (int q = warp; q < COUNT; q += W) {
                 const double t = warp_fold(lane < W ? red[q][lane] : 0.0, q < NMAX);
-                if (lane == 0) st_tagged(set + q * kPersistMaxBlocks + b, t, rnum);
+                if (lane == 0) st_tagged(set + q * kPersistMaxBlocks + b, t, mark);
             }
             // Block 0 adds them up and puts the sums in front of every block,
             // a 128-byte line each: lines polled by many blocks at once keep
@@ -490,16 +506,17 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
                     int r_[N];
 #pragma unroll
                     for (int r = 0; r < N; ++r) r_[r] = min(r * 32 + lane, nb - 1);
-                    FromTagged<double, 1>{set + q * kPersistMaxBlocks, rnum, A.limits.entry, bad}.get(r_, o);
+                    FromTagged<double, 1, true>{set + q * kPersistMaxBlocks, rnum, A.limits.entry, bad}.get(r_, o);
 #pragma unroll
                     for (int r = 0; r < N; ++r)
                         if (r * 32 + lane < nb) t = q < NMAX ? maxv(t, o[r]) : t + o[r];
                     t = warp_fold(t, q < NMAX);
-                    for (int r = lane; r < nb; r += 32) st_tagged(result + r * 8 + q, t, rnum);
+                    bad = __any_sync(0xffffffffu, bad);
+                    for (int r = lane; r < nb; r += 32) st_tagged(result + r * 8 + q, t, bad ? rnum | kFailed : rnum);
                 } else if (lane == 0) {
                     const int at_[1] = {q};
                     double o[1];
-                    FromTagged<double, 1>{result + b * 8, rnum, A.limits.entry, bad}.get(at_, o);
+                    FromTagged<double, 1, true>{result + b * 8, rnum, A.limits.entry, bad}.get(at_, o);
                     t = o[0];
                 }
                 if (lane == 0) sums[q] = t;
@@ -728,9 +745,10 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             M.r_hi[i] = (float)Q.b1;
         }
     }
-    if (b == 0 && tid == 0) {
-        S.fault = P.st->fault;
-        *P.st = S;
+    if (b == 0) {  // all but the fault, which a block sets by itself
+        constexpr int words = sizeof(DevState) / sizeof(int), skip = offsetof(DevState, fault) / sizeof(int);
+        for (int q = tid; q < words; q += nt)
+            if (q != skip) reinterpret_cast<int*>(P.st)[q] = reinterpret_cast<const int*>(&S)[q];
     }
 }
 

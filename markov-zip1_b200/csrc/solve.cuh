@@ -338,6 +338,7 @@ int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int rem, int
     A.smem_bytes = pk.smem;
     A.counter = pk.counter;
     A.limits = ctx.limits;
+    A.fail_block = ctx.fail_block;
     A.tx = pk.tx;
     A.ty = pk.ty;
     A.stage_y = pk.stage_y;

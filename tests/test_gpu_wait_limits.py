@@ -4,6 +4,7 @@ an error, and the next call on the same context is right."""
 from __future__ import annotations
 
 import ctypes as C
+import time
 from contextlib import contextmanager
 
 import numpy as np
@@ -122,4 +123,40 @@ def test_barrier_at_the_start_of_the_loop(gpu_ctx, name, iterations):
     with limits(gpu_ctx, barrier=1, entry=100):
         with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
             gpu_ctx.solve(m, o)
+    same(gpu_ctx.solve(m, o), expect)
+
+
+@pytest.mark.parametrize("polls", [1, 10])
+@pytest.mark.parametrize("iterations", [97, 40, 17, 0])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+@pytest.mark.parametrize("name", ["grid", "grid_staged"])
+def test_entry_of_another_block(gpu_ctx, name, precision, iterations, polls):
+    """The gathers of every block run out, in iterations, checks or reductions."""
+    m, o = MODELS[name](), opts(iterations, precision=Precision[precision])
+    expect = gpu_ctx.solve(m, o)
+    with limits(gpu_ctx, entry=polls):
+        with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
+            gpu_ctx.solve(m, o)
+    same(gpu_ctx.solve(m, o), expect)
+
+
+@pytest.mark.parametrize("block", [0, 1, 77])  # block 0 adds up the partials of all
+@pytest.mark.parametrize("adaptive", [True, False])  # the next reduction: the first iteration's, or the check's
+@pytest.mark.parametrize("iterations", [97, 40, 17, 0])
+@pytest.mark.parametrize("name", ["grid", "grid_staged"])
+def test_one_block_of_many(gpu_ctx, name, iterations, adaptive, block):
+    """One block's waits run out, all others' are served: the next reduction tells
+    every block, so that none goes on with a result made of stale entries nor
+    waits (for seconds, with the limits as they are) for the one that left."""
+    m, o = MODELS[name](), opts(iterations, adaptive_step_size=adaptive)
+    expect = gpu_ctx.solve(m, o)
+    lib = _lib.engine()
+    _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, block))
+    try:
+        began = time.monotonic()
+        with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
+            gpu_ctx.solve(m, o)
+        assert time.monotonic() - began < 1.0
+    finally:
+        _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, -1))
     same(gpu_ctx.solve(m, o), expect)
