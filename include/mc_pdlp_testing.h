@@ -21,8 +21,10 @@ int mc_test_inject_alloc_failures(int count);
 /* How many polls the waits inside the context's cooperative kernels take before
  * a kernel gives up and its call returns MC_ERR_CUDA: at a barrier of the grid,
  * and for one entry that another block writes.  0 restores a default (seconds).
- * A few polls make an ordinary wait run out. */
-int mc_test_set_wait_limits(mc_pdlp_ctx* ctx, unsigned barrier_polls, unsigned entry_polls);
+ * A few polls make an ordinary wait run out.  The Ruiz passes' barrier adds
+ * polls_per_nonzero (default 2) for every nonzero of the matrix. */
+int mc_test_set_wait_limits(mc_pdlp_ctx* ctx, unsigned barrier_polls, unsigned entry_polls,
+                            unsigned polls_per_nonzero);
 
 /* In the persistent loop's form of one block per SM this block behaves as if a
  * wait of its had run out before its first gather: it waits for nothing and

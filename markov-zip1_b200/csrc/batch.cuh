@@ -576,7 +576,8 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
         R.lanes = gr;
         C.lp = B.cols.lp, C.l0 = B.cols.l0, C.l1 = B.cols.l1, C.ntiles = nct;
         R.lp = B.rows.lp, R.l0 = B.rows.l0, R.l1 = B.rows.l1, R.ntiles = nrt;
-        TRY(launch_ruiz(ctx, C, R, nnz > 0 && o->ruiz_scaling ? o->ruiz_iterations : 0, 1e-3, count, partials, st));
+        TRY(launch_ruiz(ctx, C, R, nnz, nnz > 0 && o->ruiz_scaling ? o->ruiz_iterations : 0, 1e-3, count, partials,
+                        st));
     }
     Iterates<double> P;
     P.m = (int)m;

@@ -187,6 +187,7 @@ constexpr unsigned kSpinLimit = 1u << 23;  // polls of one wait (seconds) before
 struct WaitLimits {
     unsigned barrier = kSpinLimit;  // at a barrier of the whole grid
     unsigned entry = kSpinLimit;    // for one gathered entry or partial of another block
+    unsigned per_nonzero = 2;       // Ruiz: added to `barrier` for every nonzero (launch_ruiz)
 };
 
 // Barrier across the blocks of a launch, in two halves: the hardware barrier of

@@ -527,12 +527,14 @@ int mc_test_inject_alloc_failures(int count) {
     return MC_OK;
 }
 
-int mc_test_set_wait_limits(mc_pdlp_ctx* c, unsigned barrier_polls, unsigned entry_polls) {
+int mc_test_set_wait_limits(mc_pdlp_ctx* c, unsigned barrier_polls, unsigned entry_polls,
+                            unsigned polls_per_nonzero) {
     Ctx* ctx = reinterpret_cast<Ctx*>(c);
     if (!ctx) return set_error(MC_ERR_INVALID_ARGUMENT, "context is NULL");
     ctx->limits = WaitLimits{};
     if (barrier_polls) ctx->limits.barrier = barrier_polls;
     if (entry_polls) ctx->limits.entry = entry_polls;
+    ctx->limits.per_nonzero = polls_per_nonzero;
     return MC_OK;
 }
 

@@ -149,8 +149,14 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
 // ------------------------------------------------------------------ Ruiz
 // One cooperative launch (k_ruiz).  C, R: both copies, their tiles and the
 // scratch of their deltas; work: at least 6 nlp + 2 words of device memory.
-int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long passes, double tolerance, int nlp,
-                double* work, DevState* st) {
+// A block may wait at the barrier for one that has the matrix' longest line:
+// with one lane per line (the mean is short) a lane takes up to every nonzero,
+// at 0.1 us each (measured at 100,000 and 400,000 entries), so the limit grows
+// by two polls of 0.2 us or more for each.
+int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long nnz, long long passes, double tolerance,
+                int nlp, double* work, DevState* st) {
+    const unsigned limit = (unsigned)std::min<long long>(
+        UINT_MAX, ctx.limits.barrier + (long long)ctx.limits.per_nonzero * nnz);
     cudaStream_t s = ctx.stream;
     unsigned long long* errs = reinterpret_cast<unsigned long long*>(work);
     unsigned* counter = reinterpret_cast<unsigned*>(errs + 6 * (size_t)nlp);
@@ -165,7 +171,7 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long passes
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     ctx.begin_launch(MC_KERNEL_SETUP);
-    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, ctx.limits.barrier, st));
+    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, limit, st));
     ctx.end_launch();
     return ctx.launch_check("ruiz");
 }
@@ -193,7 +199,7 @@ int ruiz(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const int*
          double tolerance = 1e-3) {
     return launch_ruiz(ctx, ruiz_side_of(n, nnz, csc_start, csc_row, csc_val, col_scale, c_d0, c_d1),
                        ruiz_side_of(m, nnz, csr_start, csr_col, csr_val, row_scale, r_d0, r_d1),
-                       nnz > 0 ? passes : 0, tolerance, 1, partials, st);
+                       nnz, nnz > 0 ? passes : 0, tolerance, 1, partials, st);
 }
 
 // ------------------------------------------------------ persistent kernel

@@ -46,7 +46,7 @@ ENGINE_SIGNATURES = {
     "mc_pdlp_default_options": ([_VP], None),
     "mc_pdlp_struct_sizes": ([_VP, C.c_int], C.c_int),
     "mc_test_inject_alloc_failures": ([C.c_int], C.c_int),
-    "mc_test_set_wait_limits": ([_VP, C.c_uint, C.c_uint], C.c_int),
+    "mc_test_set_wait_limits": ([_VP, C.c_uint, C.c_uint, C.c_uint], C.c_int),
     "mc_test_fail_block": ([_VP, C.c_int], C.c_int),
     "mc_last_error": ([C.c_char_p, C.c_size_t], C.c_int),
     "mc_device_count": ([_VP], C.c_int),

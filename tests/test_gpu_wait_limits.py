@@ -28,13 +28,13 @@ MODELS = {
 
 
 @contextmanager
-def limits(ctx, barrier=0, entry=0):
+def limits(ctx, barrier=0, entry=0, per_nonzero=0):
     lib = _lib.engine()
-    _lib.check(lib.mc_test_set_wait_limits(ctx.handle, barrier, entry))
+    _lib.check(lib.mc_test_set_wait_limits(ctx.handle, barrier, entry, per_nonzero))
     try:
         yield
     finally:
-        _lib.check(lib.mc_test_set_wait_limits(ctx.handle, 0, 0))
+        _lib.check(lib.mc_test_set_wait_limits(ctx.handle, 0, 0, 2))
 
 
 def opts(iterations=97, **kw):
@@ -160,3 +160,26 @@ def test_one_block_of_many(gpu_ctx, name, iterations, adaptive, block):
     finally:
         _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, -1))
     same(gpu_ctx.solve(m, o), expect)
+
+
+def test_limit_of_the_ruiz_barrier_grows_with_the_matrix(gpu_ctx):
+    """One row with an entry in every column among short rows, which get one lane
+    each: the blocks of the short ones wait for its lane, longer the longer it is."""
+    m, n = 25_000, 100_000
+    r = np.random.default_rng(8)
+    rows = np.empty((n, 2), np.int32)
+    rows[:, 0], rows[:, 1] = 0, r.integers(1, m, n)  # 8 entries a row or fewer on average
+    some = r.random(n) < 0.9
+    start = np.concatenate([[0], np.cumsum(1 + some)])
+    keep = np.stack([np.ones(n, bool), some], 1)
+    index = rows[keep]
+    lp = mcpdlp.Model(m, n, start, index, r.uniform(0.5, 1.5, len(index)), r.normal(size=n), np.zeros(n), np.ones(n),
+                      np.full(m, -np.inf), np.full(m, 50.0))
+    assert lp.nnz < 8 * m
+    o = opts(2, ruiz_iterations=2)
+    expect = gpu_ctx.solve(lp, o)
+    with limits(gpu_ctx, barrier=2000):  # 2 ms: not enough for 100,000 entries by one lane
+        with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
+            gpu_ctx.solve(lp, o)
+    with limits(gpu_ctx, barrier=2000, per_nonzero=2):
+        same(gpu_ctx.solve(lp, o), expect)
