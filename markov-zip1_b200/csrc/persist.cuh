@@ -536,8 +536,10 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             else yn = -Q.yb;
         } else {
             const T v = add_rn(Q.y, mul_rn(Q.sigma, ax));
-            // an equality row's clamp gives its bound whatever v / sigma is
-            const T cl = Q.b0 == Q.b1 ? Q.b0 : clampv(div_recip(v, Q.sigma, Q.rsigma), Q.b0, Q.b1);
+            // an equality row's clamp gives its bound whatever v / sigma is, unless
+            // that can be 0 / 0 or inf / inf
+            const bool fixed = Q.b0 == Q.b1 && Q.rsigma > T(0) && Q.rsigma < T(INFINITY);
+            const T cl = fixed ? Q.b0 : clampv(div_recip(v, Q.sigma, Q.rsigma), Q.b0, Q.b1);
             yn = sub_rn(v, mul_rn(Q.sigma, cl));
         }
         Q.y = yn;

@@ -173,3 +173,20 @@ def test_unscaled_rows_of_any_magnitude(gpu_ctx, m, n, precision):
         ok = np.isfinite(b)
         np.testing.assert_array_equal(np.isfinite(a), ok)
         np.testing.assert_allclose(np.asarray(a)[ok], np.asarray(b)[ok], rtol=1e-11, atol=0)
+
+
+@pytest.mark.parametrize("m,n", [(40, 90), (1500, 9000)])  # cluster and grid form
+def test_equality_row_whose_step_size_is_zero(gpu_ctx, m, n):
+    """Entries whose sum overflows make the row's norm infinite and its step size
+    0: the quotient 0 / 0 is not a number in any form, an equality row's included."""
+    model = generators.random_lp(33, m, n, 5)
+    model.value[model.row_index == 3] = 1.7e308
+    assert np.count_nonzero(model.row_index == 3) > 1 and model.row_lower[3] == model.row_upper[3]
+    o = PdlpOptions(max_iterations=80, ruiz_scaling=False, adaptive_step_size=False, initial_primal_weight=1.0)
+    o.set_tolerance(1e-14)
+    res = gpu_ctx.solve(model, o)
+    assert res.extra["launches_by_kind"]["dual"] == 0
+    ref = gpu_ctx.solve_batch([model], o)[0]
+    assert ref.status == res.status == mcpdlp.PdlpStatus.numerical_failure
+    assert ref.iterations == res.iterations
+    assert np.isnan(ref.dual[3]) and np.isnan(res.dual[3])
