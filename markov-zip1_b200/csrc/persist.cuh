@@ -295,6 +295,7 @@ struct ColState {
 template <class T>
 struct RowState {
     int b = 0, e = 0;
+    bool fixed;
     T sigma, rsigma, b0, b1, y, ya, yb;  // b0, b1: row bounds, or the correction's A x_hat - b
 };
 
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
     namespace cg = cooperative_groups;
     if (tid == 0) S = *P.st;
     __syncthreads();
-    if (S.done || S.fault) return;  // every block reads the same state
+    if (S.done) return;  // every block reads the same state
     const int Gc = A.g_col, Gr = A.g_row, Gp = A.g_probe;
     const int sub_c = tid & (Gc - 1), sub_r = tid & (Gr - 1);
     // the block's lines: equal runs, at most blockDim / G of them (the launch's rule)
@@ -426,6 +427,9 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
         if (vr) {
             Q.sigma = div_rn(T(S.eta * S.omega), P.row_norm[i]);
             Q.rsigma = div_rn(T(1), Q.sigma);
+            // an equality row's clamp gives its bound whatever v / sigma is, unless
+            // that can be 0 / 0 or inf / inf
+            Q.fixed = !MX && Q.b0 == Q.b1 && Q.rsigma > T(0) && Q.rsigma < T(INFINITY);
         }
     };
     set_steps();
@@ -536,10 +540,7 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             else yn = -Q.yb;
         } else {
             const T v = add_rn(Q.y, mul_rn(Q.sigma, ax));
-            // an equality row's clamp gives its bound whatever v / sigma is, unless
-            // that can be 0 / 0 or inf / inf
-            const bool fixed = Q.b0 == Q.b1 && Q.rsigma > T(0) && Q.rsigma < T(INFINITY);
-            const T cl = fixed ? Q.b0 : clampv(div_recip(v, Q.sigma, Q.rsigma), Q.b0, Q.b1);
+            const T cl = Q.fixed ? Q.b0 : clampv(div_recip(v, Q.sigma, Q.rsigma), Q.b0, Q.b1);
             yn = sub_rn(v, mul_rn(Q.sigma, cl));
         }
         Q.y = yn;
