@@ -258,10 +258,11 @@ struct PersistArgs {
     Original O;
     Controls ctl;
     TraceBuf tr;
-    int chunks;         // whole restart chunks to run
+    int chunks;         // whole restart chunks to run, each with its check
     int R;              // iterations per chunk
-    int rem;            // iterations of a last partial chunk
-    int final_pass;     // evaluate after it (loop exhausted)
+    int skip;           // iterations of the first chunk that earlier launches ran
+    int rem;            // then the iterations of another chunk up to this one,
+    int final_pass;     // evaluated as the loop's last (1), or left for the next launch (0)
     int g_col, g_row, g_probe;  // lanes per line
     int smem_bytes;     // dynamic shared memory of the launch
     unsigned* counter;  // arrivals at the grid barrier, zeroed before the launch
@@ -557,9 +558,11 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
     for (int pass = 0; pass < passes && ok; ++pass) {
         const bool last = pass == A.chunks;  // the partial chunk and the final evaluation
         const int span = last ? A.rem : A.R;
-        int phase10 = (int)(S.iter % 10);
-        long long count = S.avg_count;
-        for (int k = 0; k < span; ++k) {
+        const int skip = pass == 0 ? A.skip : 0;
+        int phase10 = (int)((S.iter + skip) % 10);
+        long long count = S.avg_count + skip;
+        const int steps = span - skip;
+        for (int k = 0; k < steps; ++k) {
             const bool step_it = A.ctl.adaptive_step && phase10 == 0;
             phase10 = phase10 == 9 ? 0 : phase10 + 1;
             const T cnt = T((double)(++count));
@@ -646,6 +649,10 @@ __global__ void __launch_bounds__(NT, 1) k_persist(Iterates<T> P, MixedState M, 
             if (CL) bar.wait();
         }
         if (!ok) break;
+        if (last && !A.final_pass) {  // no check, and so no reduction that tells of a wait that ran out
+            if (!CL) ok = __syncthreads_or(bad) == 0;
+            break;
+        }
         // ---- the KKT check on the averages (k_residual_rows/cols[_mx], k_finalize)
         // the averages (base plus averaged correction in the mixed form) in
         // FP64, gathered by the block's lines

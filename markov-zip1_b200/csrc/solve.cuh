@@ -323,11 +323,12 @@ int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned
     return MC_OK;
 }
 
-// One launch: `chunks` whole chunks, then (with final_pass) `rem` iterations
-// and the final evaluation.
+// One launch: `chunks` whole chunks with their checks, then the iterations of
+// another chunk up to `rem`, with the final evaluation or without any.  `skip`:
+// iterations of its first chunk that earlier launches ran.
 template <class E>
-int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int rem, int final_pass, const Controls& ctl,
-                   const TraceBuf& tr) {
+int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int skip, int rem, int final_pass,
+                   const Controls& ctl, const TraceBuf& tr) {
     using T = std::remove_pointer_t<decltype(eng.P.x)>;
     const Persist& pk = eng.pk;
     PersistArgs A{};
@@ -336,6 +337,7 @@ int launch_persist(Ctx& ctx, const E& eng, int chunks, long long R, int rem, int
     A.tr = tr;
     A.chunks = chunks;
     A.R = (int)R;
+    A.skip = skip;
     A.rem = rem;
     A.final_pass = final_pass;
     A.g_col = eng.pl.g_col;
@@ -553,18 +555,37 @@ struct has_persist : std::false_type {};
 template <class E>
 struct has_persist<E, std::void_t<decltype(std::declval<E&>().pk)>> : std::true_type {};
 
-// loop_chunks on the persistent kernel: kPersistChunks chunks per launch
-// (a few milliseconds, so that a long solve is polled and never holds the
-// device in one launch), the host polling one launch behind.
-constexpr int kPersistChunks = 32;
+// Iterations of one launch of the persistent kernel (2 to 10 ms), so that a
+// long solve is polled and other work gets its turn on the device between two
+// launches: whole chunks, or parts of one that is longer than that.
+constexpr int kPersistSpan = 1280;
+
+// The iterations of a chunk up to `to` and its check (a whole chunk's, or the final evaluation).
+template <class E>
+int launch_chunk(Ctx& ctx, const E& eng, long long R, int to, int final_pass, const Controls& ctl, const TraceBuf& tr) {
+    int at = 0;
+    for (; to - at > kPersistSpan; at += kPersistSpan) {
+        TRY(launch_persist(ctx, eng, 0, R, at, at + kPersistSpan, 0, ctl, tr));
+        TRY(ctx.drain_profile());
+    }
+    TRY(launch_persist(ctx, eng, final_pass ? 0 : 1, R, at, final_pass ? to : 0, final_pass, ctl, tr));
+    return ctx.drain_profile();
+}
+
+// loop_chunks on the persistent kernel, the host polling one launch (or, above
+// kPersistSpan iterations, one chunk) behind.
 template <class E>
 int loop_persist(Ctx& ctx, const E& eng, DevState* st, ChunkLoop& L, long long stop, long long R,
                  const Controls& ctl, const TraceBuf& tr) {
     cudaStream_t s = ctx.stream;
     while (L.chunk < stop && !L.done) {
-        const int chunks = (int)std::min<long long>(stop - L.chunk, std::max<long long>(1, kPersistChunks * 40 / R));
-        TRY(launch_persist(ctx, eng, chunks, R, 0, 0, ctl, tr));
-        TRY(ctx.drain_profile());
+        const int chunks = (int)std::min<long long>(stop - L.chunk, std::max<long long>(1, kPersistSpan / R));
+        if (chunks == 1) {
+            TRY(launch_chunk(ctx, eng, R, (int)R, 0, ctl, tr));
+        } else {
+            TRY(launch_persist(ctx, eng, chunks, R, 0, 0, 0, ctl, tr));
+            TRY(ctx.drain_profile());
+        }
         L.chunk += chunks;
         L.base += chunks * R;
         if (L.have_prev) {
@@ -652,8 +673,7 @@ int finish_chunks(Ctx& ctx, const E& eng, const ChunkLoop& L, long long maxit, l
         if (rem > 0 || L.full_chunks == 0) {
             if constexpr (has_persist<E>::value) {
                 if (eng.pk.blocks > 0) {
-                    TRY(launch_persist(ctx, eng, 0, R, (int)rem, 1, ctl, tr));
-                    TRY(ctx.drain_profile());
+                    TRY(launch_chunk(ctx, eng, R, (int)rem, 1, ctl, tr));
                     CU(cudaStreamSynchronize(ctx.stream));
                     return MC_OK;
                 }

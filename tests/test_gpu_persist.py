@@ -190,3 +190,47 @@ def test_equality_row_whose_step_size_is_zero(gpu_ctx, m, n):
     assert ref.status == res.status == mcpdlp.PdlpStatus.numerical_failure
     assert ref.iterations == res.iterations
     assert np.isnan(ref.dual[3]) and np.isnan(res.dual[3])
+
+
+@pytest.mark.parametrize("m,n", [(40, 90), (2000, 9000)])  # cluster and grid form
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+def test_long_restart_periods_take_several_launches(gpu_ctx, m, n, precision):
+    """No launch runs more than 1280 iterations: a restart period of 3001 takes
+    three, and so does the rest of 2697; the iterates are the streaming kernels'."""
+    model = generators.random_lp(34, m, n, 5)
+    # no step-size rule and no restart: nothing depends on a reduction's order
+    o = PdlpOptions(max_iterations=2 * 3001 + 2697, restart_every=3001, precision=Precision[precision],
+                    adaptive_step_size=False, restart_strategy=mcpdlp.RestartStrategy.none, initial_primal_weight=1.0)
+    o.set_tolerance(1e-15)
+    res = gpu_ctx.solve(model, o)
+    assert res.extra["launches_by_kind"]["primal"] == 9
+    o.lanes_per_column, o.lanes_per_row = lanes(model.nnz / n), lanes(model.nnz / m)
+    ref = gpu_ctx.solve_batch([model], o)[0]
+    assert res.iterations == ref.iterations == 8699
+    assert rel(res.primal, ref.primal) <= 1e-11
+    assert rel(res.dual, ref.dual) <= 1e-11
+    # driven period by period: the same launches, the same result
+    s = gpu_ctx.begin(model, o)
+    while not s.iterate(1)[1]:
+        pass
+    step = s.finish()
+    np.testing.assert_array_equal(step.primal, res.primal)
+    np.testing.assert_array_equal(step.dual, res.dual)
+
+
+def test_long_restart_periods_keep_the_step_size_rule(gpu_ctx):
+    """The rule runs on every tenth iteration wherever a launch begins: a period of
+    2563 split in three against the same iterations in periods that are not, with
+    no restarts (a check that restarts nothing changes no iterate)."""
+    model = generators.random_lp(35, 300, 900, 5)
+    out = []
+    for every in (2563, 1281):
+        o = PdlpOptions(max_iterations=2562, restart_every=every, restart_strategy=mcpdlp.RestartStrategy.none)
+        o.set_tolerance(1e-300)
+        out.append(gpu_ctx.solve(model, o))
+    one_launch = PdlpOptions(max_iterations=2562, restart_every=183, restart_strategy=mcpdlp.RestartStrategy.none)
+    one_launch.set_tolerance(1e-300)
+    expect = gpu_ctx.solve(model, one_launch)
+    for r in out:
+        np.testing.assert_array_equal(r.primal, expect.primal)
+        np.testing.assert_array_equal(r.dual, expect.dual)
