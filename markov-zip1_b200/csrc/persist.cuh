@@ -133,10 +133,6 @@ struct FromTagged {
             for (int q = 0; q < N; ++q)
                 if (tag[q] != want) ld_tagged(v + (long long)STRIDE * i[q], a[q], tag[q]);
             bad = ++spins > limit;
-            if (!REDUCTION) {  // overwritten already: its owner did not wait for this block
-#pragma unroll
-                for (int q = 0; q < N; ++q) bad = bad || tag[q] > want;
-            }
         }
     }
 };

@@ -141,14 +141,14 @@ def test_entry_of_another_block(gpu_ctx, name, precision, iterations, polls):
 
 
 @pytest.mark.parametrize("block", [0, 1, 77])  # block 0 adds up the partials of all
-@pytest.mark.parametrize("adaptive", [True, False])  # the next reduction: the first iteration's, or the check's
 @pytest.mark.parametrize("iterations", [97, 40, 17, 0])
 @pytest.mark.parametrize("name", ["grid", "grid_staged"])
-def test_one_block_of_many(gpu_ctx, name, iterations, adaptive, block):
-    """One block's waits run out, all others' are served: the next reduction tells
-    every block, so that none goes on with a result made of stale entries nor
-    waits (for seconds, with the limits as they are) for the one that left."""
-    m, o = MODELS[name](), opts(iterations, adaptive_step_size=adaptive)
+def test_one_block_of_many(gpu_ctx, name, iterations, block):
+    """One block's waits run out, all others' are served: the next reduction (in the
+    first iteration, or the check without any) tells every block, so that none goes
+    on with a result made of stale entries nor waits (for seconds, with the limits
+    as they are) for the one that left."""
+    m, o = MODELS[name](), opts(iterations)
     expect = gpu_ctx.solve(m, o)
     lib = _lib.engine()
     _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, block))
@@ -157,6 +157,25 @@ def test_one_block_of_many(gpu_ctx, name, iterations, adaptive, block):
         with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
             gpu_ctx.solve(m, o)
         assert time.monotonic() - began < 1.0
+    finally:
+        _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, -1))
+    same(gpu_ctx.solve(m, o), expect)
+
+
+@pytest.mark.parametrize("block", [0, 1, 77])
+@pytest.mark.parametrize("iterations", [97, 17])
+@pytest.mark.parametrize("name", ["grid", "grid_staged"])
+def test_one_block_runs_ahead_of_the_others(gpu_ctx, name, iterations, block):
+    """Without the step-size rule's reductions the block overwrites entries that
+    others have not read: their waits run out in turn, and the call fails."""
+    m, o = MODELS[name](), opts(iterations, adaptive_step_size=False)
+    expect = gpu_ctx.solve(m, o)
+    lib = _lib.engine()
+    _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, block))
+    try:
+        with limits(gpu_ctx, entry=20_000, per_nonzero=2):
+            with pytest.raises(mcpdlp.EngineError, match=TIMED_OUT):
+                gpu_ctx.solve(m, o)
     finally:
         _lib.check(lib.mc_test_fail_block(gpu_ctx.handle, -1))
     same(gpu_ctx.solve(m, o), expect)
