@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(1024) k_sort_long_rows(const int* __restrict__
 }
 
 // ---------------------------------------------------------------------- Ruiz
-// equilibrate_model, src/scale/ruiz_scaling.cpp:167-218, all passes in one
-// cooperative launch, for one LP or for a packed batch.  Maxima are exact in
-// any order, and the rescale computes value * (delta_r[i] * delta_c[j])
+// equilibrate_model, src/scale/ruiz_scaling.cpp:167-218, all passes (up to 64)
+// in one cooperative launch, for one LP or for a packed batch.  Maxima are
+// exact in any order, and the rescale computes value * (delta_r[i] * delta_c[j])
 // exactly as :215, so the scaled matrix equals the reference's bit for bit.
 //
 // A pass reads and writes both copies of the matrix once: while a line is
@@ -340,17 +340,24 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
     flush();
 }
 
-__global__ void __launch_bounds__(kBlock) k_ruiz(RuizSide C, RuizSide R, long long passes, double tolerance, int nlp,
-                                                 unsigned long long* errs, unsigned* counter, unsigned limit,
-                                                 DevState* st) {
+// Passes [pass0, pass1); pass 0 begins with the maxima of the matrix as given.
+// counter[1] is set when there is nothing left to do after them.
+__global__ void __launch_bounds__(kBlock) k_ruiz(RuizSide C, RuizSide R, long long pass0, long long pass1,
+                                                 double tolerance, int nlp, unsigned long long* errs, unsigned* counter,
+                                                 unsigned limit, DevState* st) {
     __shared__ double scratch[32];
     BlockBarrier<false> bar{counter, 0u, limit, false};
-    ruiz_side<true>(C, nullptr, 0, errs, 0, 0, 1, nlp, tolerance, scratch);
-    ruiz_side<true>(R, nullptr, 0, errs, 0, 0, 0, nlp, tolerance, scratch);
-    int set = 0;
-    for (long long pass = 0; pass < passes; ++pass, set = set == 2 ? 0 : set + 1) {
+    if (pass0 == 0) {
+        ruiz_side<true>(C, nullptr, 0, errs, 0, 0, 1, nlp, tolerance, scratch);
+        ruiz_side<true>(R, nullptr, 0, errs, 0, 0, 0, nlp, tolerance, scratch);
+    }
+    int set = (int)(pass0 % 3);
+    for (long long pass = pass0; pass < pass1; ++pass, set = set == 2 ? 0 : set + 1) {
         if (!bar.sync()) {
-            if (threadIdx.x == 0) atomicExch(&st->fault, 1);
+            if (threadIdx.x == 0) {
+                atomicExch(&st->fault, 1);
+                atomicExch(counter + 1, 1u);
+            }
             return;
         }
         // convergence test (:185-197); a converged LP's later passes are no-ops
@@ -366,7 +373,10 @@ __global__ void __launch_bounds__(kBlock) k_ruiz(RuizSide C, RuizSide R, long lo
                 errs[(size_t)(2 * clear_set + 1) * nlp + lp] = 0ull;
             }
         }
-        if (__syncthreads_and(all)) return;
+        if (__syncthreads_and(all)) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) counter[1] = 1u;
+            return;
+        }
         const int cur = (int)(pass & 1);
         ruiz_side<false>(C, R.delta[cur], cur, errs, set, write_set, 1, nlp, tolerance, scratch);
         ruiz_side<false>(R, C.delta[cur], cur, errs, set, write_set, 0, nlp, tolerance, scratch);

@@ -147,7 +147,11 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
 }
 
 // ------------------------------------------------------------------ Ruiz
-// One cooperative launch (k_ruiz).  C, R: both copies, their tiles and the
+// Passes of one launch (40 ms at 40M nonzeros): a matrix that never converges
+// runs as many as it is given, and other work gets its turn between launches.
+constexpr int kRuizPasses = 64;
+
+// Cooperative launches of k_ruiz.  C, R: both copies, their tiles and the
 // scratch of their deltas; work: at least 6 nlp + 2 words of device memory.
 // A block may wait at the barrier for one that has the matrix' longest line:
 // with one lane per line (the mean is short) a lane takes up to every nonzero,
@@ -160,7 +164,7 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long nnz, l
     cudaStream_t s = ctx.stream;
     unsigned long long* errs = reinterpret_cast<unsigned long long*>(work);
     unsigned* counter = reinterpret_cast<unsigned*>(errs + 6 * (size_t)nlp);
-    CU(cudaMemsetAsync(work, 0, sizeof(double) * (6 * (size_t)nlp + 2), s));
+    CU(cudaMemsetAsync(work, 0, sizeof(double) * (6 * (size_t)nlp + 1), s));
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
@@ -170,9 +174,19 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long nnz, l
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    ctx.begin_launch(MC_KERNEL_SETUP);
-    CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, passes, tolerance, nlp, errs, counter, limit, st));
-    ctx.end_launch();
+    for (long long pass = 0; pass == 0 || pass < passes; pass += kRuizPasses) {
+        if (pass > 0) {
+            unsigned finished = 0;
+            CU(cudaMemcpyAsync(&finished, counter + 1, sizeof finished, cudaMemcpyDeviceToHost, s));
+            CU(cudaStreamSynchronize(s));
+            if (finished) break;
+            CU(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
+        }
+        ctx.begin_launch(MC_KERNEL_SETUP);
+        CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, pass, passes - pass > kRuizPasses ? pass + kRuizPasses : passes, tolerance,
+                              nlp, errs, counter, limit, st));
+        ctx.end_launch();
+    }
     return ctx.launch_check("ruiz");
 }
 
