@@ -748,19 +748,11 @@ int solve_batch(Ctx& ctx, const mc_lp* lps, int count, const mc_pdlp_options* o,
                                                 row_scale, stage_x, stage_y, B);
     ctx.end_launch();
     TRY(ctx.launch_check("batch unscale"));
-    // host outputs through the staging buffers (below), device outputs directly
     std::vector<Staging::Piece> x_pieces, y_pieces;
     for (int b = 0; b < count; ++b) {
-        const bool host = lps[b].memory == MC_MEMORY_HOST;
         const size_t xb = sizeof(double) * (size_t)lps[b].num_cols, yb = sizeof(double) * (size_t)lps[b].num_rows;
-        if (x_out && x_out[b] && xb) {
-            if (host) x_pieces.push_back({x_out[b], sizeof(double) * (size_t)col_off[b], xb});
-            else CU(cudaMemcpyAsync(x_out[b], stage_x + col_off[b], xb, cudaMemcpyDefault, s));
-        }
-        if (y_out && y_out[b] && yb) {
-            if (host) y_pieces.push_back({y_out[b], sizeof(double) * (size_t)row_off[b], yb});
-            else CU(cudaMemcpyAsync(y_out[b], stage_y + row_off[b], yb, cudaMemcpyDefault, s));
-        }
+        if (x_out && x_out[b] && xb) x_pieces.push_back({x_out[b], sizeof(double) * (size_t)col_off[b], xb});
+        if (y_out && y_out[b] && yb) y_pieces.push_back({y_out[b], sizeof(double) * (size_t)row_off[b], yb});
     }
     TRY(up.get(s, stage_x, x_pieces));
     TRY(up.get(s, stage_y, y_pieces));

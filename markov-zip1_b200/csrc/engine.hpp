@@ -73,6 +73,7 @@ struct Layout {
 // 6-10 us to the device and 15-20 us back, whatever its size.
 struct Staging {
     static constexpr size_t kHalf = 512u << 10;
+    static constexpr size_t kGap = 16u << 10;  // what a transfer may carry along between two pieces
     struct Piece {
         void* host;
         size_t offset, bytes;  // from the start of the device range
@@ -92,8 +93,8 @@ struct Staging {
     int flush(cudaStream_t s);
     // dst (device) <- src (host or device); ends with flush()
     int put(cudaStream_t s, void* dst, const void* src, size_t bytes);
-    // host pieces, in rising order of offset, <- device range; returns with
-    // the stream synchronised up to the copies
+    // pieces (host or device), in rising order of offset, <- device range;
+    // complete once the stream is synchronised
     int get(cudaStream_t s, const void* src, const std::vector<Piece>& pieces);
 };
 

@@ -1824,14 +1824,8 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
     for (int k = 0; k < count; ++k) {  // slot k holds variant perm[k]
         const int b = perm[k];
         const size_t xb = sizeof(double) * (size_t)n, yb = sizeof(double) * (size_t)m;
-        if (x_out && x_out[b]) {
-            if (!dev_in) x_pieces.push_back({x_out[b], (size_t)k * xb, xb});
-            else CU(cudaMemcpyAsync(x_out[b], xo + (size_t)k * n, xb, cudaMemcpyDefault, s));
-        }
-        if (y_out && y_out[b]) {
-            if (!dev_in) y_pieces.push_back({y_out[b], (size_t)k * yb, yb});
-            else CU(cudaMemcpyAsync(y_out[b], yo + (size_t)k * m, yb, cudaMemcpyDefault, s));
-        }
+        if (x_out && x_out[b]) x_pieces.push_back({x_out[b], (size_t)k * xb, xb});
+        if (y_out && y_out[b]) y_pieces.push_back({y_out[b], (size_t)k * yb, yb});
     }
     TRY(up.get(s, xo, x_pieces));
     TRY(up.get(s, yo, y_pieces));
