@@ -16,7 +16,20 @@
  * and +-INFINITY in place of BoundKind::{negative,positive}_infinity.
  *
  * Threading: calls on different contexts may run concurrently from different
- * host threads; one context must not be used by two threads at once.
+ * host threads; one context must not be used by two threads at once.  What
+ * overlaps on one GPU: an LP whose loop fits one cluster (n + m up to 4096, in
+ * the mixed form 6400) leaves the other SMs to other solves.  A larger one of up
+ * to about 57,000 columns of 8 entries takes every SM in launches of a few
+ * milliseconds; two of them fit side by side up to some 15,000 columns, beyond
+ * that they take turns.  ms per solve of 1200 iterations with 1 / 2 / 4 / 8
+ * contexts, each in its thread, and in brackets with shared_device = 1:
+ *    1000 x  3000, 18k nonzeros   5.3 / 2.7 / 1.4 / 1.3
+ *    4001 x 12007, 108k           6.9 / 4.1 / 4.2 / 4.2   (14.1 / 7.9 / 4.7 / 3.2)
+ *   10000 x 30000, 240k           7.9 / 7.4 / 7.4 / 7.4   (14.7 / 9.1 / 6.1 / 5.1)
+ *   20011 x 50021, 400k          11.3 / 10.4 / 10.4 / 10.7 (16.7 / 11.0 / 7.4 / 7.7)
+ * So four contexts or more on LPs of some 10,000 columns and up are better served
+ * with shared_device, and many LPs that are known together by
+ * mc_pdlp_ctx_solve_batch.
  * Errors: every function returns MC_OK (0) or an mc_error code; the text of
  * the last error on the calling thread is available from mc_last_error().
  * There is no CPU fallback: without a usable sm_100 device every solve
@@ -115,7 +128,12 @@ typedef struct mc_pdlp_options {
                                          of the warm start and of the cold start (x = proj(0),
                                          y = 0) on the device and run from the better one; a
                                          cold start also drops initial_primal_weight */
-    int32_t reserved_i[4];
+    int32_t shared_device;            /* 1: several contexts solve on this GPU at the same time
+                                         (see Threading above): LPs too large for one cluster
+                                         run in kernels that overlap with other solves.
+                                         0: the fastest form for a solve alone.  The two
+                                         agree up to rounding */
+    int32_t reserved_i[3];
     double reserved_d[8];
 } mc_pdlp_options;
 

@@ -270,10 +270,13 @@ inline cudaLaunchConfig_t persist_config(const Ctx& ctx, const Persist& pk, cuda
 //   * for a short x-bar (rows gather few columns: 30000 x 3000 took 12 us
 //     against 10.6), and
 //   * for rows of so few entries that one lane takes a row: its trips to L2
-//     then follow one another (60000 x 50000, 5 per row: 18 us against 11).
+//     then follow one another (60000 x 50000, 5 per row: 18 us against 11), and
+//   * where the caller shares the device (option shared_device): it takes every
+//     SM, so that solves of other contexts wait for its launches.
 constexpr int kClusterVector64 = 4096, kClusterVector32 = 6400;  // n + m
 template <class T>
-int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned* counter, void* tagged, Persist* out) {
+int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned* counter, void* tagged, bool shared,
+                 Persist* out) {
     *out = Persist{};
     int dev_smem = 0;
     CU(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
@@ -312,7 +315,7 @@ int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned
         }
     }
     const int nb = ctx.sm_count;
-    if (tagged && nb <= kPersistMaxBlocks && lanes_of(nb) <= kGridThreadsWide && pl.g_row >= 2 &&
+    if (tagged && !shared && nb <= kPersistMaxBlocks && lanes_of(nb) <= kGridThreadsWide && pl.g_row >= 2 &&
         (double)n * nb > 2.0 * (double)nnz) {
         Persist pk;
         pk.blocks = nb;
@@ -1062,7 +1065,7 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         eng.O = O;
         eng.pl = make_plan<double>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
         TRY(plan_persist<double>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
-                            o_tagged ? at(o_tagged) : nullptr, &eng.pk));
+                            o_tagged ? at(o_tagged) : nullptr, o->shared_device != 0, &eng.pk));
         TRY(choose_start(ctx, eng, st, ctl, have_warm, o->warm_start_guard != 0, start, [] { return MC_OK; }, res));
     } else {
         EngineMixed& eng = SS.emx;
@@ -1146,7 +1149,7 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         eng.O = O;
         eng.pl = make_plan<float>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
         TRY(plan_persist<float>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
-                            o_tagged ? at(o_tagged) : nullptr, &eng.pk));
+                            o_tagged ? at(o_tagged) : nullptr, o->shared_device != 0, &eng.pk));
         // the FP32 dual kernel has no block partials: one block per kBlock/G rows
         // (about 40 waves) lets the block scheduler even out the last wave,
         // 13% faster on B200 than one resident wave; the FP64 and primal

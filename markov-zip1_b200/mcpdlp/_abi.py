@@ -84,7 +84,8 @@ class McPdlpOptions(C.Structure):
         ("lanes_per_column", C.c_int32),
         ("lanes_per_row", C.c_int32),
         ("warm_start_guard", C.c_int32),
-        ("reserved_i", C.c_int32 * 4),
+        ("shared_device", C.c_int32),
+        ("reserved_i", C.c_int32 * 3),
         ("reserved_d", C.c_double * 8),
     ]
 
