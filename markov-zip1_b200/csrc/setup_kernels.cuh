@@ -128,10 +128,13 @@ __global__ void k_scatter_rows(int n, const int* __restrict__ col_start, const i
     }
 }
 
-constexpr int kShortRow = 32;     // rows up to this length: a warp sorts them in registers
+constexpr int kShortRow = 32;     // rows up to this length: sorted by a warp in registers, or by one thread
 constexpr int kSmemSortRow = 4096;  // rows up to this length: shared-memory bitonic sort
 
-// Sorts short rows by column and lists the long rows for the block-level sort.
+// Sort short rows by column and list the long rows for the block-level sort:
+// by a warp per row, or (k_sort_short_rows_thread) by a thread per row where the
+// rows fill the chip's threads and are short (build_csr has the rule).
+//
 // A warp per row, an entry per lane: the row is read once, each entry counts
 // the smaller ones by shuffles and goes to that place.  (An insertion sort by
 // one thread per row is a chain of dependent loads and stores: 51 us for 1000
@@ -160,6 +163,31 @@ __global__ void k_sort_short_rows(int m, const int* __restrict__ row_start, int*
     if (in) {
         col_index[b + place] = key;
         value[b + place] = v;
+    }
+}
+
+// An entry moves down past the larger ones before it.
+__global__ void k_sort_short_rows_thread(int m, const int* __restrict__ row_start, int* __restrict__ col_index,
+                                         double* __restrict__ value, int* __restrict__ long_rows,
+                                         int* __restrict__ long_count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const int b = row_start[i], e = row_start[i + 1];
+    if (e - b > kShortRow) {
+        long_rows[atomicAdd(long_count, 1)] = i;
+        return;
+    }
+    for (int p = b + 1; p < e; ++p) {
+        const int key = col_index[p];
+        const double v = value[p];
+        int q = p;
+        for (; q > b && col_index[q - 1] > key; --q) {
+            col_index[q] = col_index[q - 1];
+            value[q] = value[q - 1];
+        }
+        if (q == p) continue;
+        col_index[q] = key;
+        value[q] = v;
     }
 }
 

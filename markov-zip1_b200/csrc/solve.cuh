@@ -117,8 +117,17 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
     ctx.begin_launch(MC_KERNEL_SETUP);
     k_scatter_rows<<<nb_n, kBlock, 0, s>>>(n, csc_start, csc_row, csc_val, csr_start, cursor, csr_col, csr_val);
     ctx.end_launch();
+    // A warp per row pays per row, a thread per row for the length of the chain
+    // (the whole transpose, us, thread / warp): 16M nonzeros in rows of 2 on
+    // average 2860 / 3850, of 4 2110 / 2590, of 8 1930 / 2090, of 16 1970 / 1850; 2M
+    // in rows of 2 620 / 705, of 6 (333,000 rows) 638 / 645, of 8 (250,000) 640 / 628.
     ctx.begin_launch(MC_KERNEL_SETUP);
-    k_sort_short_rows<<<(int)(((long long)m * 32 + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, csr_start, csr_col, csr_val, long_rows, counters);
+    if (m >= 2048LL * ctx.sm_count && nnz <= 8LL * m)
+        k_sort_short_rows_thread<<<(m + kBlock - 1) / kBlock, kBlock, 0, s>>>(m, csr_start, csr_col, csr_val, long_rows,
+                                                                             counters);
+    else
+        k_sort_short_rows<<<(int)(((long long)m * 32 + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, csr_start, csr_col,
+                                                                                             csr_val, long_rows, counters);
     ctx.end_launch();
     ctx.begin_launch(MC_KERNEL_SETUP);
     k_max_line<<<blocks_for(ctx, m, kBlock), kBlock, 0, s>>>(m, csr_start, counters + 1);
