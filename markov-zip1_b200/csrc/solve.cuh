@@ -277,12 +277,27 @@ inline cudaLaunchConfig_t persist_config(const Ctx& ctx, const Persist& pk, cuda
 // everyone polls, so a short y is copied to shared memory by each block
 // (stage_y), and it is left out
 //   * for a short x-bar (rows gather few columns: 30000 x 3000 took 12 us
-//     against 10.6), and
+//     against 10.6),
 //   * for rows of so few entries that one lane takes a row: its trips to L2
-//     then follow one another (60000 x 50000, 5 per row: 18 us against 11), and
+//     then follow one another (60000 x 50000, 5 per row: 18 us against 11),
+//   * for FP32 with one entry in most columns of very many and more rows than can
+//     be copied (8000 x 113000 14 us against 10), and
 //   * where the caller shares the device (option shared_device): it takes every
 //     SM, so that solves of other contexts wait for its launches.
 constexpr int kClusterVector64 = 4096, kClusterVector32 = 6400;  // n + m
+
+// Whether each block copies y: when that is at most `copy` loads per entry
+// gathered.  Where most columns have one entry, many columns poll the same y and
+// the copy pays further (one entry a column, us per iteration without / with the
+// copy: 2000 x 113000 14.8 / 8.5 FP64 and 18.8 / 7.7 FP32, 1600 x 70000 12.0 /
+// 7.2, 5000 x 113000 FP32 12.2 / 8.6; but 2000 x 30000 6.3 / 7.0).
+template <class T>
+bool persist_stage_y(int m, int n, long long nnz, int blocks, long long lanes) {
+    const bool single = (double)nnz < 1.5 * n;
+    const double copy = !single || lanes <= 352 ? 2.0 : sizeof(T) == 4 && lanes > 600 ? 8.0 : 6.0;
+    return m * (double)blocks <= copy * (double)nnz && 2.0 * m * sizeof(T) <= 65536.0;
+}
+
 template <class T>
 int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned* counter, void* tagged, bool shared,
                  Persist* out) {
@@ -338,7 +353,8 @@ int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned
         PersistKernel<T> gk = pk.threads <= kGridThreads ? k_persist<T, false, kGridThreads>
                                                          : k_persist<T, false, kGridThreadsWide>;
         CU(cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, top));
-        pk.stage_y = m * (double)nb <= 2.0 * (double)nnz && 2.0 * m * sizeof(T) <= 65536.0;
+        pk.stage_y = persist_stage_y<T>(m, n, nnz, nb, lanes_of(nb));
+        if (sizeof(T) == 4 && (double)nnz < 1.5 * n && lanes_of(nb) > 600 && !pk.stage_y) return MC_OK;
         pk.smem = (int)need(nb, pk.stage_y ? 2.0 * m * sizeof(T) : 0.0);
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gk, pk.threads, (size_t)pk.smem) == cudaSuccess &&
