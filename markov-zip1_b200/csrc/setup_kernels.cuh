@@ -14,13 +14,19 @@ __global__ void k_fill(T* __restrict__ a, long long n, T v) {
         a[i] = v;
 }
 
-// max row length (for the long-row sort path)
-__global__ void k_max_line(int lines, const int* __restrict__ start, int* __restrict__ out) {
-    int mx = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < lines; i += gridDim.x * blockDim.x)
-        mx = max(mx, start[i + 1] - start[i]);
-    for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+// longest row (for the long-row sort path) and longest column
+__global__ void k_max_line(int m, const int* __restrict__ row_start, int n, const int* __restrict__ col_start,
+                           int* __restrict__ longest) {
+    int mx[2] = {0, 0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+        mx[0] = max(mx[0], row_start[i + 1] - row_start[i]);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        mx[1] = max(mx[1], col_start[j + 1] - col_start[j]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        for (int off = 16; off > 0; off >>= 1) mx[q] = max(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], off));
+        if ((threadIdx.x & 31) == 0) atomicMax(longest + q, mx[q]);
+    }
 }
 
 // ---------------------------------------------------------------- validation

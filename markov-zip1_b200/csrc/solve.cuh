@@ -74,7 +74,8 @@ Plan make_plan(const Ctx& ctx, int m, int n, long long nnz, int force_col, int f
 
 // ------------------------------------------------------------- transpose
 // CSR(A) from CSC(A): count, scan, scatter, per-row sort (ascending column,
-// so the layout and every SpMV over it are run-to-run deterministic).
+// so the layout and every SpMV over it are run-to-run deterministic).  On the
+// way, where asked for, the entries of the longest row and column.
 // In-place inclusive scan of data[0..len), multi-level over tile totals; tmp
 // holds (len + 1) / kScanTile + 4096 ints.
 void inclusive_scan(Ctx& ctx, int* data, long long len, int* tmp, int kind = MC_KERNEL_SETUP) {
@@ -101,11 +102,12 @@ void inclusive_scan(Ctx& ctx, int* data, long long len, int* tmp, int kind = MC_
 
 int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const int* csc_row,
               const double* csc_val, int* csr_start, int* csr_col, double* csr_val, int* cursor,
-              int* long_rows, int* counters /*[2]*/, int* scan_tmp) {
+              int* long_rows, int* counters /*[3]*/, int* scan_tmp, int* longest = nullptr) {
     cudaStream_t s = ctx.stream;
+    if (longest) longest[0] = longest[1] = 0;
     CU(cudaMemsetAsync(csr_start, 0, sizeof(int) * (size_t)(m + 1), s));
     CU(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)m, s));
-    CU(cudaMemsetAsync(counters, 0, sizeof(int) * 2, s));
+    CU(cudaMemsetAsync(counters, 0, sizeof(int) * 3, s));
     if (nnz > 0) {
         ctx.begin_launch(MC_KERNEL_SETUP);
         k_count_rows<<<blocks_for(ctx, nnz, kBlock) * 4, kBlock, 0, s>>>(nnz, csc_row, csr_start);
@@ -130,12 +132,16 @@ int build_csr(Ctx& ctx, int m, int n, long long nnz, const int* csc_start, const
                                                                                              csr_val, long_rows, counters);
     ctx.end_launch();
     ctx.begin_launch(MC_KERNEL_SETUP);
-    k_max_line<<<blocks_for(ctx, m, kBlock), kBlock, 0, s>>>(m, csr_start, counters + 1);
+    k_max_line<<<blocks_for(ctx, std::max(m, n), kBlock), kBlock, 0, s>>>(m, csr_start, n, csc_start, counters + 1);
     ctx.end_launch();
-    int host_counters[2] = {0, 0};
+    int host_counters[3] = {0, 0, 0};
     CU(cudaMemcpyAsync(host_counters, counters, sizeof host_counters, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     TRY(ctx.drain_profile());
+    if (longest) {
+        longest[0] = host_counters[1];
+        longest[1] = host_counters[2];
+    }
     if (host_counters[0] > 0) {
         int* tmp_col = nullptr;
         double* tmp_val = nullptr;
@@ -280,8 +286,7 @@ inline cudaLaunchConfig_t persist_config(const Ctx& ctx, const Persist& pk, cuda
 //     against 10.6),
 //   * for rows of so few entries that one lane takes a row: its trips to L2
 //     then follow one another (60000 x 50000, 5 per row: 18 us against 11),
-//   * for FP32 with one entry in most columns of very many and more rows than can
-//     be copied (8000 x 113000 14 us against 10), and
+//   * for long lines (persist_lines), and
 //   * where the caller shares the device (option shared_device): it takes every
 //     SM, so that solves of other contexts wait for its launches.
 constexpr int kClusterVector64 = 4096, kClusterVector32 = 6400;  // n + m
@@ -298,9 +303,35 @@ bool persist_stage_y(int m, int n, long long nnz, int blocks, long long lanes) {
     return m * (double)blocks <= copy * (double)nnz && 2.0 * m * sizeof(T) <= 65536.0;
 }
 
+// Whether the grid form takes lines as long as the longest.  A group of lanes
+// has its line for the whole launch, four entries per lane in a step; while one
+// works through a long line everybody else polls what it will write, and a step
+// takes 1.0 to 1.5 us against 0.6 in the streaming kernels.  us per iteration, grid
+// / streaming, FP64 (FP32 is worse by the streaming kernels' gain):
+//   4000 x 12000, 6 a column, and 20 rows of 128 (8 steps)  12.4 / 15.3
+//                                         of 256 (16)       22.2 / 19.6
+//                                         of 1200 (75)      87 / 55
+//   25000 x 50000, 8 a column, 20 rows of 5000 (625)        950 / 193
+//   3000 x 30000, 3 a column, 20 columns of 64 (16)         21.8 / 19.7
+//   5000 x 40000, 1 a column, 20 columns of 32 (8)          21.9 / 13.9
+//   transport 20 x 500 (16, 20k nonzeros)                   10.2 / 21.7
+// With y in shared memory the columns cost little (2000 x 90000 with a full
+// column 93 / 220) and nobody polls a row's y: 1000 x 30000, rows of 1500 (25
+// steps) 19.5 / 25, 50 x 2000 transport (31) 42 / 33; smaller ones lose little
+// where they lose at all (1000 x 12000, rows of 5000 (80) 54 / 59; 3000 x 12000
+// with 20 full rows (188) 163 / 133).
 template <class T>
-int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned* counter, void* tagged, bool shared,
-                 Persist* out) {
+bool persist_lines(const Plan& pl, int m, int n, long long nnz, const int* longest, bool stage_y, long long lanes) {
+    const double row_steps = longest[0] / (4.0 * pl.g_row), col_steps = longest[1] / (4.0 * pl.g_col);
+    if (stage_y) return row_steps <= (n + m <= 15000 ? 192.0 : 24.0);
+    // one entry a column, too many rows to copy (8000 x 113000 FP32 14 us against 10)
+    if (sizeof(T) == 4 && (double)nnz < 1.5 * n && lanes > 600) return false;
+    return row_steps <= (nnz <= 35000 ? 16.0 : 8.0) && col_steps <= 4.0;
+}
+
+template <class T>
+int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, const int* longest, unsigned* counter,
+                 void* tagged, bool shared, Persist* out) {
     *out = Persist{};
     int dev_smem = 0;
     CU(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
@@ -354,7 +385,7 @@ int plan_persist(Ctx& ctx, const Plan& pl, int m, int n, long long nnz, unsigned
                                                          : k_persist<T, false, kGridThreadsWide>;
         CU(cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, top));
         pk.stage_y = persist_stage_y<T>(m, n, nnz, nb, lanes_of(nb));
-        if (sizeof(T) == 4 && (double)nnz < 1.5 * n && lanes_of(nb) > 600 && !pk.stage_y) return MC_OK;
+        if (!persist_lines<T>(pl, m, n, nnz, longest, pk.stage_y, lanes_of(nb))) return MC_OK;
         pk.smem = (int)need(nb, pk.stage_y ? 2.0 * m * sizeof(T) : 0.0);
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gk, pk.threads, (size_t)pk.smem) == cudaSuccess &&
@@ -1016,9 +1047,10 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
 
     // ---- setup (FP64, both forms)
     CU(cudaMemsetAsync(st, 0, sizeof(DevState), s));
+    int longest[2];  // entries of a row, of a column
     TRY(build_csr(ctx, m, n, nnz, csc_start, csc_row, csc_val, csr_start, csr_col, csr_val,
                   static_cast<int*>(at(o_cursor)), static_cast<int*>(at(o_long)), counters,
-                  static_cast<int*>(at(o_scan))));
+                  static_cast<int*>(at(o_scan)), longest));
     TRY(ruiz(ctx, m, n, nnz, csc_start, csc_row, csc_val, csr_start, csr_col, csr_val, row_scale, col_scale,
              ax_bar, row_norm, dx, col_norm, partials, st, o->ruiz_scaling ? o->ruiz_iterations : 0));
     const double obj_sign = (lp->objective_sense == MC_MAXIMIZE) ? -1.0 : 1.0;
@@ -1089,7 +1121,7 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         P.st = st;
         eng.O = O;
         eng.pl = make_plan<double>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
-        TRY(plan_persist<double>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
+        TRY(plan_persist<double>(ctx, eng.pl, m, n, nnz, longest, static_cast<unsigned*>(at(o_counter)),
                             o_tagged ? at(o_tagged) : nullptr, o->shared_device != 0, &eng.pk));
         TRY(choose_start(ctx, eng, st, ctl, have_warm, o->warm_start_guard != 0, start, [] { return MC_OK; }, res));
     } else {
@@ -1173,7 +1205,7 @@ int begin_session(Ctx& ctx, const mc_lp* lp, const mc_pdlp_options* o, const dou
         M.yb = f_yb;
         eng.O = O;
         eng.pl = make_plan<float>(ctx, m, n, nnz, o->lanes_per_column, o->lanes_per_row);
-        TRY(plan_persist<float>(ctx, eng.pl, m, n, nnz, static_cast<unsigned*>(at(o_counter)),
+        TRY(plan_persist<float>(ctx, eng.pl, m, n, nnz, longest, static_cast<unsigned*>(at(o_counter)),
                             o_tagged ? at(o_tagged) : nullptr, o->shared_device != 0, &eng.pk));
         // the FP32 dual kernel has no block partials: one block per kBlock/G rows
         // (about 40 waves) lets the block scheduler even out the last wave,

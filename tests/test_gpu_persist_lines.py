@@ -38,3 +38,40 @@ def test_one_entry_a_column(gpu_ctx, m, n, fp64, fp32):
     model = generators.random_lp(70, m, n, 1)
     assert takes_the_loop(gpu_ctx, model, "fp64") == fp64
     assert takes_the_loop(gpu_ctx, model, "fp32_refine") == fp32
+
+
+def with_long_lines(m, n, k, row=0, col=0):
+    """k entries a column at random rows but the first, which has `row` entries;
+    the first column has `col` in all."""
+    r = np.random.default_rng(m + n + row + col)
+    entries = {(int(i), j): r.normal() for j in range(n) for i in 1 + r.choice(m - 1, size=k, replace=False)}
+    for j in range(1, 1 + min(row, n - 1)):
+        entries[(0, j)] = r.normal()
+    more = [i for i in range(1, m) if (i, 0) not in entries][:max(0, col - k)]
+    for i in more:
+        entries[(i, 0)] = r.normal()
+    i, j = np.array(list(entries)).T
+    order = np.lexsort((i, j))
+    i, j, v = i[order], j[order], np.array(list(entries.values()))[order]
+    x = np.where(r.random(n) < 0.3, 0.0, r.uniform(0.1, 5.0, n))
+    b = np.bincount(i, weights=v * x[j], minlength=m)
+    return mcpdlp.Model(m, n, np.concatenate([[0], np.cumsum(np.bincount(j, minlength=n))]), i, v, r.normal(size=n),
+                        np.zeros(n), np.full(n, 10.0), b, b)
+
+
+# steps are of four entries per lane; lanes from the mean: 4 a row and 1 a column, 32 a row where it has 200
+@pytest.mark.parametrize("shape,row,col,loop", [
+    ((4000, 12000, 6), 128, 0, True), ((4000, 12000, 6), 129, 0, False),     # 8 steps
+    ((4000, 12000, 6), 0, 16, True), ((4000, 12000, 6), 0, 17, False),       # 4 steps
+    ((1000, 6000, 4), 256, 0, True), ((1000, 6000, 4), 257, 0, False),       # few nonzeros: 16 steps
+    ((600, 20000, 6), 3072, 0, True), ((600, 20000, 6), 3073, 0, False),     # the dual copied: 24 steps
+    ((600, 20000, 6), 0, 500, True),                                         # and columns of any length
+    ((1000, 12000, 8), 11999, 0, True)])                                     # and few lines: 192 steps
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+def test_longest_lines(gpu_ctx, shape, row, col, loop, precision):
+    model = with_long_lines(*shape, row=row, col=col)
+    if row:
+        assert np.bincount(model.row_index).max() == row
+    if col:
+        assert np.diff(model.col_start).max() == col
+    assert takes_the_loop(gpu_ctx, model, precision) == loop
