@@ -30,6 +30,7 @@ namespace mc {
 constexpr int kVarWarps = kBlock / 32;  // warps per block, one line each per trip
 constexpr int kVarGathers = 4;          // gathers in flight per lane (split_dot)
 constexpr int kVarDualBlocks = 2;       // blocks per SM of the split dual kernels
+constexpr int kVarLongColumn = 64;      // longest column above which kv_primal_wide asks for indices ahead (pack_dot)
 
 // The base LP (scaled, shared by every variant).
 struct VarBase {
@@ -340,7 +341,11 @@ __device__ __forceinline__ void pack_window(const int* __restrict__ idx, const T
 }
 // AHEAD (rows): the indices of the next window are asked for before the
 // gathers of this one are waited for: dual 18.7 -> 14.1 us (128 variants, FP32).
-// Columns rarely fill one window, and the registers cost a block per SM.
+// Columns rarely fill one window, and the registers cost a block per SM; but a
+// long one is a chain of windows, and all others wait for it, so FP64 columns
+// are asked for ahead where the longest has more than kVarLongColumn entries: 120
+// iterations of 4 variants of 2000 x 6000 with a column of 256 entries 7.5 -> 4.4 ms
+// (7.2 with a warp per line), with one of 64 3.6 -> 2.9, of 32 2.95 either way.
 template <bool AHEAD, class T>
 __device__ __forceinline__ Pack<T> pack_dot(int b, int e, const int* __restrict__ idx, const T* __restrict__ val,
                                             const T* __restrict__ v, int Kp, unsigned long long pol) {
@@ -532,6 +537,7 @@ struct DualLane {
 };
 
 // the primal step of an iteration without a probe (kv_primal_step has the formulas)
+template <bool AHEAD>
 __global__ void __launch_bounds__(kBlock) kv_primal_wide(VarBase Bs, VarRefs V, int lg, int kk) {
     const VarPack<double> me(V, lg, kk, false);
     if (!me.any) return;
@@ -543,7 +549,7 @@ __global__ void __launch_bounds__(kBlock) kv_primal_wide(VarBase Bs, VarRefs V, 
         const double cn = __ldg(Bs.col_norm + j), cj = __ldg(Bs.c + j);
         Pack<double> x = ld_pack(V.x + q), xa = ld_pack(V.xa + q);
         const Pack<double> lo = ld_pack(V.lo + q), hi = ld_pack(V.hi + q);
-        Pack<double> xb = pack_dot<false>(b, e, Bs.ri, Bs.cv, V.y + me.k, V.Kp, pol);
+        Pack<double> xb = pack_dot<AHEAD>(b, e, Bs.ri, Bs.cv, V.y + me.k, V.Kp, pol);
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             const double g = __dadd_rn(cj, xb.v[w]);
@@ -941,7 +947,7 @@ struct EngineVariants {
     dim3 grid;
     WideGrid cols, wide;  // packs of columns, of rows
     dim3 rows;
-    bool rows_wide;
+    bool rows_wide, long_cols;
     int shape_class(const DevState&) const { return 0; }
     void use_class(int) const {}
 
@@ -949,7 +955,8 @@ struct EngineVariants {
         cudaStream_t s = ctx.stream;
         ctx.begin_launch(MC_KERNEL_PRIMAL);
         if (step) kv_primal_step<<<grid, kBlock, 0, s>>>(Bs, V, k);
-        else kv_primal_wide<<<cols.grid, kBlock, 0, s>>>(Bs, V, cols.lg, k);
+        else if (long_cols) kv_primal_wide<true><<<cols.grid, kBlock, 0, s>>>(Bs, V, cols.lg, k);
+        else kv_primal_wide<false><<<cols.grid, kBlock, 0, s>>>(Bs, V, cols.lg, k);
         ctx.end_launch();
         if (step) {
             ctx.begin_launch(MC_KERNEL_DUAL_STEP);
@@ -1626,8 +1633,9 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
 
     // ---- the base LP's setup (shared by every variant)
     CU(cudaMemsetAsync(st, 0, sizeof(DevState) * (count + 2), s));
+    int longest[2];  // entries of a row, of a column
     TRY(build_csr(ctx, m, n, nnz, cs, ri, cv, rs, ci, rv, static_cast<int*>(at(o_cursor)),
-                  static_cast<int*>(at(o_long)), counters, static_cast<int*>(at(o_scan))));
+                  static_cast<int*>(at(o_long)), counters, static_cast<int*>(at(o_scan)), longest));
     TRY(ruiz(ctx, m, n, nnz, cs, ri, cv, rs, ci, rv, row_scale, col_scale, y_scratch, row_norm, x_scratch,
              col_norm, part1, st,
              o->ruiz_scaling ? o->ruiz_iterations : 0));
@@ -1736,7 +1744,9 @@ int solve_variants(Ctx& ctx, const mc_lp* base, int count, const double* const* 
         eng.V = V;
         eng.O = O;
         eng.grid = grid;
-        eng.cols = wide_grid<double>(ctx, kv_primal_wide, n, Kp);
+        eng.long_cols = longest[1] > kVarLongColumn;
+        eng.cols = eng.long_cols ? wide_grid<double>(ctx, kv_primal_wide<true>, n, Kp)
+                                 : wide_grid<double>(ctx, kv_primal_wide<false>, n, Kp);
         eng.rows = dual_grid(ctx, kv_dual<false>, m, groups);
         eng.wide = wide_grid<double>(ctx, kv_dual_wide<false>, m, Kp);
         eng.rows_wide = rows_wide;
