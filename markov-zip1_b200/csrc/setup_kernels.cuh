@@ -272,6 +272,12 @@ __global__ void __launch_bounds__(1024) k_sort_long_rows(const int* __restrict__
 // request per entry, which bounds the pass: 0.26 ms per copy at 40M nonzeros).
 // Before, a pass was seven launches with a thread per line: per call 12.9 ms
 // of rescales and 1.7 ms of maxima at 40M nonzeros, 350 us at 600.
+// A short line is one chain start -> index -> delta -> value, so its last one to
+// three entries go together and three blocks share an SM (mc_ruiz_equilibrate, 10
+// passes, ms, seven launches / two blocks and entry by entry / now: rows of 1 on
+// average, 3M x 1M 1.77 / 2.95 / 2.25, rows of 0.8, 10M x 4M 5.7 / 10.0 / 7.2; rows
+// of 20, 2M x 5M 16.4 / 11.1 / 9.2).  At four blocks it spills: 8.8 for the last,
+// but 0.98 against 0.90 for rows of 1600.
 struct RuizSide {
     const int* start;
     const int* inner;
@@ -308,13 +314,25 @@ __device__ __forceinline__ double ruiz_line(const RuizSide& S, const double* __r
 #pragma unroll
         for (int q = 0; q < 4; ++q) mx = maxv(mx, fabs(v[q]));
     }
-    for (; p < e; p += G) {
-        double v = ld_stream(S.value + p);
-        if (!FIRST) {
-            v = __dmul_rn(v, __dmul_rn(dout, __ldcg(delta_in + ld_stream(S.inner + p))));
-            st_stream(S.value + p, v);
+    if (p < e) {  // the last one to three, together
+        double v[3], d[3];
+        bool in[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            in[q] = p + q * G < e;
+            v[q] = in[q] ? ld_stream(S.value + p + q * G) : 0.0;
         }
-        mx = maxv(mx, fabs(v));
+        if (!FIRST) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) d[q] = in[q] ? __ldcg(delta_in + ld_stream(S.inner + p + q * G)) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                v[q] = __dmul_rn(v[q], __dmul_rn(dout, d[q]));
+                if (in[q]) st_stream(S.value + p + q * G, v[q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mx = in[q] ? maxv(mx, fabs(v[q])) : mx;
     }
     for (int off = G >> 1; off > 0; off >>= 1) mx = maxv(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     return mx;
@@ -376,9 +394,9 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
 
 // Passes [pass0, pass1); pass 0 begins with the maxima of the matrix as given.
 // counter[1] is set when there is nothing left to do after them.
-__global__ void __launch_bounds__(kBlock) k_ruiz(RuizSide C, RuizSide R, long long pass0, long long pass1,
-                                                 double tolerance, int nlp, unsigned long long* errs, unsigned* counter,
-                                                 unsigned limit, DevState* st) {
+__global__ void __launch_bounds__(kBlock, 3) k_ruiz(RuizSide C, RuizSide R, long long pass0, long long pass1,
+                                                    double tolerance, int nlp, unsigned long long* errs,
+                                                    unsigned* counter, unsigned limit, DevState* st) {
     __shared__ double scratch[32];
     BlockBarrier<false> bar{counter, 0u, limit, false};
     if (pass0 == 0) {
