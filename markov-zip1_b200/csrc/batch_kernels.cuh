@@ -242,15 +242,7 @@ __global__ void kb_step_size(const double* __restrict__ partials, BatchRefs B, C
     const int r0 = B.rows.first[lp], r1 = B.rows.first[lp + 1];
     const double dxn = reduce_partials(partials + SLOT_DX * kMaxTiles + c0, c1 - c0, scratch, OpSum());
     const double adx = reduce_partials(partials + SLOT_ADX * kMaxTiles + r0, r1 - r0, scratch, OpSum());
-    if (threadIdx.x == 0 && ctl.adaptive_step && dxn > 1e-14 && adx > 1e-14) {
-        const double L = sqrt(adx / dxn);
-        if (L > 1e-6) {
-            const double target = 0.95 / L;
-            const double eta = st->eta;
-            if (target < eta) st->eta = maxv(0.1, maxv(target, eta * 0.8));
-            else if (target > 1.05 * eta && eta < 0.99) st->eta = minv(0.99, eta * 1.05);
-        }
-    }
+    if (threadIdx.x == 0 && ctl.adaptive_step) st->eta = next_eta(st->eta, dxn, adx);
 }
 
 __global__ void __launch_bounds__(kBlock) kb_dual_apply(Iterates<double> P, BatchRefs B, int k) {

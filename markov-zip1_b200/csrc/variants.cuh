@@ -211,15 +211,7 @@ __global__ void kv_step_size(VarRefs V, Controls ctl) {
     if (st->done) return;
     const double dxn = reduce_partials(var_partial(V, SLOT_DX, k), V.nb, scratch, OpSum());
     const double adx = reduce_partials(var_partial(V, SLOT_ADX, k), V.nb, scratch, OpSum());
-    if (threadIdx.x == 0 && ctl.adaptive_step && dxn > 1e-14 && adx > 1e-14) {
-        const double L = sqrt(adx / dxn);
-        if (L > 1e-6) {
-            const double target = 0.95 / L;
-            const double eta = st->eta;
-            if (target < eta) st->eta = maxv(0.1, maxv(target, eta * 0.8));
-            else if (target > 1.05 * eta && eta < 0.99) st->eta = minv(0.99, eta * 1.05);
-        }
-    }
+    if (threadIdx.x == 0 && ctl.adaptive_step) st->eta = next_eta(st->eta, dxn, adx);
 }
 
 // ---------------------------------------------------------- pack kernels
