@@ -117,8 +117,16 @@ typedef struct mc_pdlp_options {
     int32_t precision;                /* MC_PRECISION_FP64 */
     int32_t device;                   /* CUDA ordinal used by mc_pdlp_solve, default 0 */
     int32_t profile_kernels;          /* 1: time every kernel launch with CUDA events
-                                         (no CUDA graph; slower); fills kernel_ms_by_kind */
-    int32_t check_every_chunks;       /* host status poll interval in restart chunks, default 1 */
+                                         (no CUDA graph; slower); fills kernel_ms_by_kind.
+                                         An LP whose loop is one kernel (small and medium
+                                         LPs, see Threading) has all of it, duals and
+                                         checks too, under MC_KERNEL_PRIMAL; its per-kernel
+                                         split exists with shared_device = 1 for LPs beyond
+                                         one cluster only */
+    int32_t check_every_chunks;       /* host status poll interval in restart chunks, default 1;
+                                         no effect on an LP whose loop is one kernel: it is
+                                         polled once per launch (1280 iterations, or one
+                                         restart period where that is longer) */
     int32_t lanes_per_column;         /* A^T y kernel: 0 = automatic (single LP: by mean
                                          column length; batch: the lanes autotuner, timed on
                                          the batch and kept per context and batch shape),
@@ -138,8 +146,8 @@ typedef struct mc_pdlp_options {
 } mc_pdlp_options;
 
 enum {
-    MC_KERNEL_PRIMAL = 0,    /* A^T y SpMV + primal prox + averages; small LPs: the
-                                persistent kernel (whole restart chunks)      */
+    MC_KERNEL_PRIMAL = 0,    /* A^T y SpMV + primal prox + averages; small and medium
+                                LPs: the persistent kernel (the whole loop)   */
     MC_KERNEL_DUAL = 1,      /* A x-bar SpMV + dual prox + averages           */
     MC_KERNEL_DUAL_STEP = 2, /* A x-bar and A dx SpMV on step-size iterations */
     MC_KERNEL_RESIDUAL = 3,  /* KKT residual SpMVs + reductions + restart     */
