@@ -272,12 +272,16 @@ __global__ void __launch_bounds__(1024) k_sort_long_rows(const int* __restrict__
 // request per entry, which bounds the pass: 0.26 ms per copy at 40M nonzeros).
 // Before, a pass was seven launches with a thread per line: per call 12.9 ms
 // of rescales and 1.7 ms of maxima at 40M nonzeros, 350 us at 600.
-// A short line is one chain start -> index -> delta -> value, so its last one to
-// three entries go together and three blocks share an SM (mc_ruiz_equilibrate, 10
-// passes, ms, seven launches / two blocks and entry by entry / now: rows of 1 on
-// average, 3M x 1M 1.77 / 2.95 / 2.25, rows of 0.8, 10M x 4M 5.7 / 10.0 / 7.2; rows
-// of 20, 2M x 5M 16.4 / 11.1 / 9.2).  At four blocks it spills: 8.8 for the last,
-// but 0.98 against 0.90 for rows of 1600.
+// A short line is one chain start -> index -> delta -> value, so the chain is what
+// a pass waits for: a line's last one to three entries go together, the next
+// line's ends and delta come meanwhile, and where both sides have a thread a line
+// (SHORT: fewer than 8 entries on average) the lanes are a constant and four blocks
+// share an SM.  mc_ruiz_equilibrate, 10 passes, ms, seven launches a pass / the
+// general form entry by entry / now: rows of 1 on average, 3M x 1M 1.84 / 2.95 / 1.77;
+// rows of 0.8, 10M x 4M 5.64 / 10.0 / 5.74; seven launches / now: rows of 3, 1M x 3M
+// 1.85 / 1.77; of 4, 2M x 2M 2.99 / 2.51; of 7 4.58 / 3.80; of 20, 2M x 5M 16.1 / 10.4.
+// The first four in the general form of now 1.99, 6.7, 1.96 and 2.65; in windows
+// of two entries at six blocks an SM 2.43, 7.7, 2.58 and 5.2.
 struct RuizSide {
     const int* start;
     const int* inner;
@@ -290,51 +294,44 @@ struct RuizSide {
     int ntiles, lines, per;
 };
 
+// W entries of a line from p, those before e, together: rescaled, and the
+// maximum of |a|.
+template <bool FIRST, int W, bool ALL>
+__device__ __forceinline__ double ruiz_window(const RuizSide& S, const double* __restrict__ delta_in, double dout, int p,
+                                              int e, int G, double mx) {
+    double v[W];
+    bool in[W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        in[q] = ALL || p + q * G < e;
+        v[q] = in[q] ? ld_stream(S.value + p + q * G) : 0.0;
+    }
+    if (!FIRST) {
+        double d[W];
+#pragma unroll
+        for (int q = 0; q < W; ++q) d[q] = in[q] ? __ldcg(delta_in + ld_stream(S.inner + p + q * G)) : 0.0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            v[q] = __dmul_rn(v[q], __dmul_rn(dout, d[q]));
+            if (in[q]) st_stream(S.value + p + q * G, v[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < W; ++q) mx = in[q] ? maxv(mx, fabs(v[q])) : mx;
+    return mx;
+}
+
 // Entries [b, e) of line j: maximum of |a| after this pass' rescale.
-template <bool FIRST>
+template <bool FIRST, bool SHORT>
 __device__ __forceinline__ double ruiz_line(const RuizSide& S, const double* __restrict__ delta_in, double dout, int b,
                                             int e, int sub) {
-    const int G = S.lanes;
+    const int G = SHORT ? 1 : S.lanes;
     double mx = 0.0;
     int p = b + sub;
-    for (; p + 3 * G < e; p += 4 * G) {
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = ld_stream(S.value + p + q * G);
-        if (!FIRST) {
-            double d[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) d[q] = __ldcg(delta_in + ld_stream(S.inner + p + q * G));
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                v[q] = __dmul_rn(v[q], __dmul_rn(dout, d[q]));
-                st_stream(S.value + p + q * G, v[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) mx = maxv(mx, fabs(v[q]));
-    }
-    if (p < e) {  // the last one to three, together
-        double v[3], d[3];
-        bool in[3];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            in[q] = p + q * G < e;
-            v[q] = in[q] ? ld_stream(S.value + p + q * G) : 0.0;
-        }
-        if (!FIRST) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) d[q] = in[q] ? __ldcg(delta_in + ld_stream(S.inner + p + q * G)) : 0.0;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                v[q] = __dmul_rn(v[q], __dmul_rn(dout, d[q]));
-                if (in[q]) st_stream(S.value + p + q * G, v[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 3; ++q) mx = in[q] ? maxv(mx, fabs(v[q])) : mx;
-    }
-    for (int off = G >> 1; off > 0; off >>= 1) mx = maxv(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    for (; p + 3 * G < e; p += 4 * G) mx = ruiz_window<FIRST, 4, true>(S, delta_in, dout, p, e, G, mx);
+    if (p < e) mx = ruiz_window<FIRST, 3, false>(S, delta_in, dout, p, e, G, mx);
+    if (!SHORT)
+        for (int off = G >> 1; off > 0; off >>= 1) mx = maxv(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     return mx;
 }
 
@@ -347,13 +344,13 @@ __device__ __forceinline__ bool ruiz_converged(const unsigned long long* errs, i
     return r < tolerance && c < tolerance;
 }
 
-template <bool FIRST>
+template <bool FIRST, bool SHORT>
 __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta_in, int cur, unsigned long long* errs,
                                           int read_set, int write_set, int side, int nlp, double tolerance,
                                           double* scratch) {
-    const int G = S.lanes, sub = threadIdx.x & (G - 1);
-    const double* own = S.delta[cur];
-    double* next = S.delta[FIRST ? cur : cur ^ 1];
+    const int G = SHORT ? 1 : S.lanes, sub = threadIdx.x & (G - 1);
+    const double* own = cur ? S.delta[1] : S.delta[0];
+    double* next = (FIRST ? cur : !cur) ? S.delta[1] : S.delta[0];
     double err = 0.0;
     int lp = 0;
     auto flush = [&]() {
@@ -362,9 +359,40 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
             atomicMax(errs + (size_t)(2 * write_set + side) * nlp + lp, (unsigned long long)__double_as_longlong(err));
         err = 0.0;
     };
+    // line j with maximum mx: the next pass' delta
+    auto finish = [&](int j, double mx, double dout) {
+        if (mx == 0.0) mx = 1.0;
+        next[j] = 1.0 / sqrt(mx);
+        err = maxv(err, fabs(1.0 - mx));
+        S.scale[j] = FIRST ? 1.0 : S.scale[j] * dout;
+    };
+    if (!S.lp) {  // one LP: the next line's ends and delta come while this line's entries do
+        const int step = (int)gridDim.x * S.per;
+        int j = (int)blockIdx.x * S.per + (int)threadIdx.x / G, b = 0, e = 0;
+        double dout = 1.0;
+        if (j < S.lines) {
+            b = __ldg(S.start + j);
+            e = __ldg(S.start + j + 1);
+            if (!FIRST) dout = own[j];
+        }
+        for (int t = blockIdx.x; t < S.ntiles; t += gridDim.x) {
+            const int jn = t + (int)gridDim.x < S.ntiles ? j + step : S.lines;
+            int bn = 0, en = 0;
+            double dn = 1.0;
+            if (jn < S.lines) {
+                bn = __ldg(S.start + jn);
+                en = __ldg(S.start + jn + 1);
+                if (!FIRST) dn = own[jn];
+            }
+            const double mx = ruiz_line<FIRST, SHORT>(S, delta_in, dout, b, e, sub);
+            if (j < S.lines && sub == 0) finish(j, mx, dout);
+            j = jn, b = bn, e = en, dout = dn;
+        }
+        flush();
+        return;
+    }
     for (int t = blockIdx.x; t < S.ntiles; t += gridDim.x) {
-        const int l0 = S.lp ? S.l0[t] : t * S.per, l1 = S.lp ? S.l1[t] : min(S.lines, l0 + S.per);
-        const int tile_lp = S.lp ? S.lp[t] : 0;
+        const int l0 = S.l0[t], l1 = S.l1[t], tile_lp = S.lp[t];
         if (tile_lp != lp) {
             flush();
             lp = tile_lp;
@@ -380,13 +408,8 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
                 e = __ldg(S.start + j + 1);
                 if (!FIRST) dout = own[j];
             }
-            double mx = ruiz_line<FIRST>(S, delta_in, dout, b, e, sub);
-            if (valid && sub == 0) {
-                if (mx == 0.0) mx = 1.0;
-                next[j] = 1.0 / sqrt(mx);
-                err = maxv(err, fabs(1.0 - mx));
-                S.scale[j] = FIRST ? 1.0 : S.scale[j] * dout;
-            }
+            const double mx = ruiz_line<FIRST, SHORT>(S, delta_in, dout, b, e, sub);
+            if (valid && sub == 0) finish(j, mx, dout);
         }
     }
     flush();
@@ -394,14 +417,15 @@ __device__ __forceinline__ void ruiz_side(const RuizSide& S, const double* delta
 
 // Passes [pass0, pass1); pass 0 begins with the maxima of the matrix as given.
 // counter[1] is set when there is nothing left to do after them.
-__global__ void __launch_bounds__(kBlock, 3) k_ruiz(RuizSide C, RuizSide R, long long pass0, long long pass1,
-                                                    double tolerance, int nlp, unsigned long long* errs,
-                                                    unsigned* counter, unsigned limit, DevState* st) {
+template <bool SHORT>
+__global__ void __launch_bounds__(kBlock, SHORT ? 4 : 3)
+    k_ruiz(RuizSide C, RuizSide R, long long pass0, long long pass1, double tolerance, int nlp,
+           unsigned long long* errs, unsigned* counter, unsigned limit, DevState* st) {
     __shared__ double scratch[32];
     BlockBarrier<false> bar{counter, 0u, limit, false};
     if (pass0 == 0) {
-        ruiz_side<true>(C, nullptr, 0, errs, 0, 0, 1, nlp, tolerance, scratch);
-        ruiz_side<true>(R, nullptr, 0, errs, 0, 0, 0, nlp, tolerance, scratch);
+        ruiz_side<true, SHORT>(C, nullptr, 0, errs, 0, 0, 1, nlp, tolerance, scratch);
+        ruiz_side<true, SHORT>(R, nullptr, 0, errs, 0, 0, 0, nlp, tolerance, scratch);
     }
     int set = (int)(pass0 % 3);
     for (long long pass = pass0; pass < pass1; ++pass, set = set == 2 ? 0 : set + 1) {
@@ -430,8 +454,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_ruiz(RuizSide C, RuizSide R, long
             return;
         }
         const int cur = (int)(pass & 1);
-        ruiz_side<false>(C, R.delta[cur], cur, errs, set, write_set, 1, nlp, tolerance, scratch);
-        ruiz_side<false>(R, C.delta[cur], cur, errs, set, write_set, 0, nlp, tolerance, scratch);
+        ruiz_side<false, SHORT>(C, cur ? R.delta[1] : R.delta[0], cur, errs, set, write_set, 1, nlp, tolerance, scratch);
+        ruiz_side<false, SHORT>(R, cur ? C.delta[1] : C.delta[0], cur, errs, set, write_set, 0, nlp, tolerance, scratch);
     }
 }
 

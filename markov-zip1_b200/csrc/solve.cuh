@@ -180,11 +180,13 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long nnz, l
     unsigned long long* errs = reinterpret_cast<unsigned long long*>(work);
     unsigned* counter = reinterpret_cast<unsigned*>(errs + 6 * (size_t)nlp);
     CU(cudaMemsetAsync(work, 0, sizeof(double) * (6 * (size_t)nlp + 1), s));
+    // a thread a line on both sides (the times are at k_ruiz)
+    const auto kernel = C.lanes == 1 && R.lanes == 1 ? k_ruiz<true> : k_ruiz<false>;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid_for(ctx, k_ruiz, std::max(C.ntiles, R.ntiles), 1));
+    cfg.gridDim = dim3((unsigned)grid_for(ctx, kernel, std::max(C.ntiles, R.ntiles), 1));
     cfg.blockDim = dim3(kBlock);
     cfg.stream = s;
     cfg.attrs = &attr;
@@ -198,8 +200,8 @@ int launch_ruiz(Ctx& ctx, const RuizSide& C, const RuizSide& R, long long nnz, l
             CU(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
         }
         ctx.begin_launch(MC_KERNEL_SETUP);
-        CU(cudaLaunchKernelEx(&cfg, k_ruiz, C, R, pass, passes - pass > kRuizPasses ? pass + kRuizPasses : passes, tolerance,
-                              nlp, errs, counter, limit, st));
+        const long long last = passes - pass > kRuizPasses ? pass + kRuizPasses : passes;
+        CU(cudaLaunchKernelEx(&cfg, kernel, C, R, pass, last, tolerance, nlp, errs, counter, limit, st));
         ctx.end_launch();
     }
     return ctx.launch_check("ruiz");
