@@ -83,9 +83,9 @@ class PdlpOptions:
     lanes_per_column: int = 0                      # SpMV tuning, 0 = chosen by line length
     lanes_per_row: int = 0
     warm_start_guard: bool = False                 # run from the better of warm / cold start
-    shared_device: bool = False                    # several contexts solve on the GPU at once
     initial_primal: Optional[np.ndarray] = None   # warm start, original space
     initial_dual: Optional[np.ndarray] = None
+    shared_device: bool = False                    # several contexts solve on the GPU at once
 
     def set_tolerance(self, tol: float) -> None:
         """pdlp.hpp:35-39"""
